@@ -271,6 +271,7 @@ struct Tables {
   std::vector<int> zd, zm;
   std::vector<int> et;        // [nmat+1]
   std::vector<double> ep;     // [(nmat+1)*6]
+  std::vector<int> el_off;    // [ninst+1] first element of each mesh
 };
 
 int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void* const* dh,
@@ -375,6 +376,9 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
     return cuda_fail(error, r, "bl_init");
   }
   cudaError_t st = cudaSuccess;
+  int *d_exl = nullptr, *d_moff = nullptr, nex = 0;  // the edges (k_edge_refs)
+  std::vector<int> moff = T ? T->el_off : std::vector<int>{0, nel};
+  const int nmesh = (int)moff.size() - 1;
   bl::DevFields& F = x->F;
   F.nel = nel;
   F.nnd = nnd;
@@ -458,6 +462,20 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
       su::k_sort<<<gn, su::kThreads, 0, x->stream>>>(d_off, nullptr, nel, nnd, d_ent2);
       F.ne_off = d_off;
       F.ne_ent = d_ent2;
+    }
+    // the edges' slots, for the build that computes an edge once; how many
+    // there are is known at the next wait
+    if (fp_mode == BL_FP_FAST) {
+      uint4* d_er = dalloc<uint4>(x, nel, st);
+      d_exl = dalloc<int>(x, 2L * nel, st);
+      d_moff = dalloc<int>(x, nmesh + 1, st);
+      int* d_nex = dalloc<int>(x, 1, st);
+      if (st != cudaSuccess) goto fail;
+      up(x, d_moff, moff.data(), nmesh + 1);
+      su::k_edge_refs<<<ge, su::kThreads, 0, x->stream>>>(d_nd, d_ee, d_fc, d_it, nel, d_moff,
+                                                          nmesh, d_er, d_exl, d_nex);
+      cudaMemcpyAsync(&nex, d_nex, sizeof(int), cudaMemcpyDeviceToHost, x->stream);
+      F.eref = d_er;
     }
     r = cudaGetLastError();
     if (r != cudaSuccess) {
@@ -671,7 +689,21 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
     C.eos_ggm1 = d_g2;
     cudaStreamSynchronize(x->stream);
   }
+  if (fp_mode == BL_FP_FAST) {
+    namespace su = bl::setup;
+    F.nslot = 2 * nel + nex;
+    int4* d_en = dalloc<int4>(x, F.nslot, st);
+    int4* d_eq = dalloc<int4>(x, F.nslot, st);
+    F.erec = dalloc<d4>(x, F.nslot, st);
+    F.esqx = dalloc<double>(x, F.nslot, st);
+    if (st != cudaSuccess) goto fail;
+    su::k_edge_slots<<<su::blocks_for(F.nslot, su::kThreads), su::kThreads, 0, x->stream>>>(
+        F.ielnd, F.ielel, F.ielfc, F.indtype, nel, d_moff, nmesh, d_exl, F.nslot, d_en, d_eq);
+    F.es_n = d_en;
+    F.es_q = d_eq;
+  }
   r = cudaStreamSynchronize(x->stream);
+  if (r == cudaSuccess) r = cudaGetLastError();
   if (r != cudaSuccess) {
     st = r;
     goto fail;
@@ -1398,6 +1430,7 @@ int bl_init_batch(bl_ctx** out, int ninst, const bl_sizes* sizes, const bl_confi
       for (int k = 0; k < BL_NEOSPARAM; k++) T.ep.push_back(c.eos_param[m][k]);
     }
   }
+  T.el_off = el_off;
   bl_config C = c0;
   int rc = init_impl(out, &S, &C, cdh.data(), fp_mode, error, &T);
   if (rc != BL_SUCCESS) return rc;

@@ -116,6 +116,15 @@ struct DevFields {
   d4 *fcdv, *fcdm, *eflux, *cndm, *cnflux, *cnfu, *cnfv, *cnm0, *cnmass_new;
   double *vpr, *mpr, *cutm_el;
   double* rscr25;            // split-advection stale-scratch emulation (unused)
+  // edges (fast build; bl_setup.cuh): slots of unique edges, each
+  // with its nodes, elements and the edges that continue it, and each
+  // element's four slots
+  int nslot, nslot_pad;
+  const int4* es_n;          // [nslot] nodes a, b, element, element across
+  const int4* es_q;          // [nslot] continuing edges' nodes, or codes < 0
+  const uint4* eref;         // [nel] 2*slot + (1: run the other way) of each face
+  d4* erec;                  // [nslot] what k_edge leaves for the two elements
+  double* esqx;              // [nslot] squared length
   // dt reduction partials
   double* red_v;             // [2*nblk]
   int* red_i;                // [2*nblk]

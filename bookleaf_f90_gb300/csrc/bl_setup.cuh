@@ -205,5 +205,201 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
+// ---------------------------------------------------------------- edges
+//
+// The edge viscosity's limiter of a face compares the face with the two
+// faces that continue it across the element's neighbouring sides
+// (hydro_kn_edgeviscosity.f90:117-183).  On most meshes the two elements
+// that share a face see the same continuing faces, so its limiter, edge
+// coefficient and lengths are the same from both sides; they are then
+// computed once, in a slot of that edge.  A face 0 or 3 always has a slot
+// of its own (nel + nel); a face 1 or 2 uses the slot of the face across it
+// when that is a face 0 or 3 with the same nodes, the same two elements and
+// the same two continuing faces, whichever way round, and otherwise gets an
+// extra slot.  Any mesh the range checks accept is covered: a face whose
+// two sides disagree simply has two slots.
+//
+// The slots of the faces 0 run along the direction that crosses faces 1 and
+// 3 where the mesh's numbering has a constant stride S that way (the first
+// element's neighbour across face 1, if S divides the mesh): slot
+// j * (n / S) + i for element i * S + j.  The faces 3 run along the
+// element numbers.  In both, an edge and the one that continues it then
+// take adjacent slots on meshes numbered along mesh lines, which k_edge
+// shares between adjacent threads; where they do not, the table holds the
+// continuing face's nodes instead.
+enum : int { kEndWall = -1, kEndMirror = -2, kEndAdjacent = -3 };
+
+__device__ __forceinline__ int at4(const int4& v, int j) {
+  return j == 0 ? v.x : (j == 1 ? v.y : (j == 2 ? v.z : v.w));
+}
+__device__ __forceinline__ int face_byte(int packed, int j) { return (packed >> (8 * j)) & 3; }
+
+// the nodes of the two faces that continue face f of element e, or the
+// boundary rule's ratio there (kEndWall: 0, kEndMirror: 1) in both entries
+struct EdgeEnds {
+  int p1, q1, p2, q2;
+};
+__device__ __forceinline__ EdgeEnds edge_ends(const int4* nd, const int4* ee, const int* fc,
+                                              const int* it, int e, int f) {
+  const int4 n = nd[e], nb = ee[e];
+  const int fcp = fc[e];
+  const int s = (f & 1) ? 0 : 1;            // the neighbours across sides s and s + 2
+  const bool first = f == 3 || f == 0;
+  const int in1 = at4(nb, s), in2 = at4(nb, s + 2);
+  const int f1 = face_byte(fcp, s), f2 = face_byte(fcp, s + 2);
+  EdgeEnds r;
+  if (in1 == e) {
+    const bool m = it[at4(n, s)] < 0 && it[at4(n, (s + 1) & 3)] < 0 && in2 != e;
+    r.p1 = r.q1 = m ? kEndMirror : kEndWall;
+  } else {
+    const int4 m = nd[in1];
+    const int k = (f1 + (first ? 1 : 3)) & 3;
+    r.p1 = at4(m, k);
+    r.q1 = at4(m, (k + 1) & 3);
+  }
+  if (in2 == e) {
+    const bool m = it[at4(n, s + 2)] < 0 && it[at4(n, (s + 3) & 3)] < 0 && in1 != e;
+    r.p2 = r.q2 = m ? kEndMirror : kEndWall;
+  } else {
+    const int4 m = nd[in2];
+    const int k = (f2 + (first ? 3 : 1)) & 3;
+    r.p2 = at4(m, k);
+    r.q2 = at4(m, (k + 1) & 3);
+  }
+  return r;
+}
+
+// the mesh of element or slot i: the last one that begins at or before it
+__device__ __forceinline__ int mesh_at(const int* moff, int nmesh, int i) {
+  int lo = 0, hi = nmesh - 1;
+  while (lo < hi) {
+    const int m = (lo + hi + 1) >> 1;
+    if (moff[m] <= i) lo = m;
+    else hi = m - 1;
+  }
+  return lo;
+}
+// the slots of a mesh's faces 0: n elements from off, stride S (1: in order)
+struct SlotMap {
+  int off, n, S;
+};
+__device__ __forceinline__ SlotMap slot_map(const int* moff, int nmesh, const int4* ee, int i) {
+  const int m = mesh_at(moff, nmesh, i);
+  SlotMap r;
+  r.off = moff[m];
+  r.n = moff[m + 1] - r.off;
+  r.S = ee[r.off].y - r.off;
+  if (r.S < 2 || r.S >= r.n || r.n % r.S != 0) r.S = 1;
+  return r;
+}
+__device__ __forceinline__ int slot_of(const SlotMap& r, int e) {
+  const int l = e - r.off;
+  return r.S == 1 ? e : r.off + (l % r.S) * (r.n / r.S) + l / r.S;
+}
+__device__ __forceinline__ int element_of(const SlotMap& r, int slot) {
+  const int p = slot - r.off, R = r.n / r.S;
+  return r.S == 1 ? slot : r.off + (p % R) * r.S + p / R;
+}
+
+// Each element's four slots; the faces that need an extra one go to exl
+// (4 * element + face) in any order, counted in *nex.
+__global__ void __launch_bounds__(kThreads)
+    k_edge_refs(const int4* __restrict__ nd, const int4* __restrict__ ee,
+                const int* __restrict__ fc, const int* __restrict__ it, int nel,
+                const int* __restrict__ moff, int nmesh, uint4* __restrict__ er,
+                int* __restrict__ exl, int* __restrict__ nex) {
+  const int e = blockIdx.x * kThreads + threadIdx.x;
+  if (e >= nel) return;
+  const SlotMap sm = slot_map(moff, nmesh, ee, e);
+  unsigned ref[4];
+  ref[0] = 2u * (unsigned)slot_of(sm, e);
+  ref[3] = 2u * ((unsigned)nel + (unsigned)e);
+  const int4 n = nd[e], nb = ee[e];
+  const int fcp = fc[e];
+  for (int f = 1; f <= 2; f++) {
+    const int w = at4(nb, f), g = face_byte(fcp, f);
+    const int a = at4(n, f), b = at4(n, f + 1);
+    bool same = false, rev = false;
+    if (w != e && (g == 0 || g == 3) && at4(ee[w], g) == e && face_byte(fc[w], g) == f) {
+      const int4 m = nd[w];
+      const int c = at4(m, g), d = at4(m, (g + 1) & 3);
+      rev = a == d && b == c;
+      if (rev || (a == c && b == d)) {
+        const EdgeEnds x = edge_ends(nd, ee, fc, it, e, f);
+        EdgeEnds y = edge_ends(nd, ee, fc, it, w, g);
+        if (rev) {
+          int t = y.p1;
+          y.p1 = y.q1;
+          y.q1 = t;
+          t = y.p2;
+          y.p2 = y.q2;
+          y.q2 = t;
+        }
+        same = (x.p1 == y.p1 && x.q1 == y.q1 && x.p2 == y.p2 && x.q2 == y.q2) ||
+               (x.p1 == y.p2 && x.q1 == y.q2 && x.p2 == y.p1 && x.q2 == y.q1);
+      }
+    }
+    if (same) {
+      const unsigned slot = g == 3 ? (unsigned)nel + (unsigned)w
+                                   : (unsigned)slot_of(slot_map(moff, nmesh, ee, w), w);
+      ref[f] = 2u * slot + (rev ? 1u : 0u);
+    } else {
+      const int k = atomicAdd(nex, 1);
+      exl[k] = 4 * e + f;
+      ref[f] = 2u * (2u * (unsigned)nel + (unsigned)k);
+    }
+  }
+  er[e] = make_uint4(ref[0], ref[1], ref[2], ref[3]);
+}
+
+// The slots' tables: en = (node a, node b, element, element across), eq =
+// the continuing faces' nodes (p1, q1, p2, q2), with kEndAdjacent in p1
+// where the first is the edge of the slot before and in p2 where the second
+// is that of the slot after (the two ends change places if that makes them
+// so: the limiter is symmetric in them).
+__global__ void __launch_bounds__(kThreads)
+    k_edge_slots(const int4* __restrict__ nd, const int4* __restrict__ ee,
+                 const int* __restrict__ fc, const int* __restrict__ it, int nel,
+                 const int* __restrict__ moff, int nmesh, const int* __restrict__ exl, int nslot,
+                 int4* __restrict__ en, int4* __restrict__ eq) {
+  const int slot = blockIdx.x * kThreads + threadIdx.x;
+  if (slot >= nslot) return;
+  int e, f, ep = -1, ex = -1;  // the elements of the slots before and after
+  if (slot < 2 * nel) {
+    f = slot < nel ? 0 : 3;
+    const int k = slot < nel ? slot : slot - nel;
+    const SlotMap sm = slot_map(moff, nmesh, ee, k);
+    e = f == 0 ? element_of(sm, k) : k;
+    if (k > sm.off) ep = f == 0 ? element_of(sm, k - 1) : k - 1;
+    if (k + 1 < sm.off + sm.n) ex = f == 0 ? element_of(sm, k + 1) : k + 1;
+  } else {
+    const int v = exl[slot - 2 * nel];
+    e = v >> 2;
+    f = v & 3;
+  }
+  const int4 n = nd[e];
+  EdgeEnds r = edge_ends(nd, ee, fc, it, e, f);
+  auto is_edge = [&](int el, int p, int q) {
+    if (el < 0) return false;
+    const int4 m = nd[el];
+    return p == at4(m, f) && q == at4(m, (f + 1) & 3);
+  };
+  bool before1 = is_edge(ep, r.p1, r.q1), before2 = is_edge(ep, r.p2, r.q2);
+  bool after1 = is_edge(ex, r.p1, r.q1), after2 = is_edge(ex, r.p2, r.q2);
+  if (!before1 && !after2 && (before2 || after1)) {
+    const EdgeEnds o = r;
+    r.p1 = o.p2;
+    r.q1 = o.q2;
+    r.p2 = o.p1;
+    r.q2 = o.q1;
+    before1 = before2;
+    after2 = after1;
+  }
+  if (before1) r.p1 = kEndAdjacent;
+  if (after2) r.p2 = kEndAdjacent;
+  en[slot] = make_int4(at4(n, f), at4(n, (f + 1) & 3), e, at4(ee[e], f));
+  eq[slot] = make_int4(r.p1, r.q1, r.p2, r.q2);
+}
+
 }  // namespace setup
 }  // namespace bl

@@ -73,15 +73,6 @@ static __device__ __noinline__ double dsqrt_call(double x) { return dsqrt_rn(x);
 #ifndef BL_GETDT_MINB
 #define BL_GETDT_MINB 7
 #endif
-// The fast build's k_getdt as two kernels (BL_GETDT_SPLIT): the edge
-// viscosity, then the dt scans and reduction.  Measured on Sedov 512x512:
-// the same step time in FP64 (293.6-294.0 against 293.6-293.8 us), 4-5 %
-// faster in the demoted form (k_getdt 62.1 against 68.7-71.0 us; 205.1
-// against 215.0 us per step), which is latency-bound and whose halves run
-// without spills; the build enables it for the demoted form only.
-#ifndef BL_GETDT_SPLIT
-#define BL_GETDT_SPLIT 0
-#endif
 // The fast build may also use exact algebraic identities that can change
 // only the sign of a zero (negation symmetry of opposite corners); the
 // exact build evaluates every expression as written.
@@ -602,11 +593,8 @@ __device__ __forceinline__ void getdt_div(const DevFields& F, int iel, const dou
   }
 }
 
-// hydro_dr_getcs2 (elcs2 += elvisc; mixed cells: sum frmass*(cpcs2+cpvisc))
-// and the element's CFL candidate from its squared length len
-// (getdt_cfl_len)
-__device__ __forceinline__ void getdt_cfl(const DevFields& F, int iel, double len, double visc,
-                                          double& cflv, int& cfli) {
+// hydro_dr_getcs2: elcs2 += elvisc; mixed cells: sum frmass*(cpcs2+cpvisc)
+__device__ __forceinline__ double signal_speed(const DevFields& F, int iel, double visc) {
   double cs2v = F.cs2[iel] + visc;
   const int imx = F.elmx ? F.elmx[iel] : -1;
   if (imx >= 0) {
@@ -616,6 +604,13 @@ __device__ __forceinline__ void getdt_cfl(const DevFields& F, int iel, double le
     cs2v = w1;
   }
   F.cs2v[iel] = cs2v;
+  return cs2v;
+}
+
+// the element's CFL candidate from its squared length len (getdt_cfl_len)
+__device__ __forceinline__ void getdt_cfl(const DevFields& F, int iel, double len, double visc,
+                                          double& cflv, int& cfli) {
+  const double cs2v = signal_speed(F, iel, visc);
 #if BL_MIXED
   const double r11 = len < 0.0 ? DBL_MAX : from_lr(DIV(to_lr(len), to_lr(cs2v)));
 #else
@@ -802,12 +797,12 @@ __device__ __forceinline__ void getdt_finish(const DevFields& F, const DevCfg& C
 }
 
 #if BL_FAST_ALGEBRA
-// Fast build.  The quantities of a face that both elements sharing it
-// compute -- its lengths, unit vectors and the inverse ratio of its
-// projections -- from the face's velocity (du, dv) and position (dx, dy)
-// differences; the face vectors' projections on their own unit vectors
-// are |d|^2 / max(|d|, zerocut) (exact in real arithmetic, never negative,
-// so the reference's sign guards drop out).
+// The quantities of a face that both elements sharing it compute -- its
+// lengths, unit vectors and the inverse ratio of its projections -- from
+// the face's velocity (du, dv) and position (dx, dy) differences; the face
+// vectors' projections on their own unit vectors are |d|^2 / max(|d|,
+// zerocut) (exact in real arithmetic, never negative, so the reference's
+// sign guards drop out).
 // (in lr: FP64, or FP32 in the mixed build)
 struct FaceQ {
   lr du, dv, lu, lx, uh, vh, xh, yh, w1;
@@ -841,8 +836,8 @@ __device__ __forceinline__ lr nb_ratio(const FaceQ& f, lr ddx, lr ddy, lr ddu, l
   return q * f.w1;
 #endif
 }
-
-// k_getdt of the fast build shares face work between neighbouring threads.
+#if BL_MIXED
+// k_getdt of the mixed build shares face work between neighbouring threads.
 // A block of BS threads takes BS - 2 consecutive elements; thread t holds
 // element blockIdx*(BS-2) + t - 1, so threads 0 and BS-1 hold the
 // neighbours of the block's first and last elements (halos).  Every
@@ -858,11 +853,15 @@ __device__ __forceinline__ lr nb_ratio(const FaceQ& f, lr ddx, lr ddy, lr ddu, l
 // generated meshes elements are numbered along mesh lines, so the face
 // across face 2 and the two limiter neighbours of side 0 are the adjacent
 // elements and take the shared path.
-// PART 0 is the whole kernel; with BL_GETDT_SPLIT the launch runs PART 1,
-// the edge viscosity (elvisc and the corner forces), then PART 2, which
-// reads elvisc back for the CFL and divergence candidates and the dt
-// reduction (the same blocks over the same elements in both).
-template <int BS, bool BATCH, int PART = 0>
+// Launched twice: PART 1, the edge viscosity (elvisc and the corner
+// forces), then PART 2, which reads elvisc back for the CFL and divergence
+// candidates and the dt reduction (the same blocks over the same elements
+// in both); neither half spills, and the pair takes 62.1 us on Sedov
+// 512x512 against 68.7-71.0 us in one kernel.  The FP64 build's form, one
+// thread per edge of the mesh (k_edge), would take 59 us here, but FP32
+// rounds each of an edge's two sides its own way: it would change results
+// in the seventh digit, so the element form stays.
+template <int BS, bool BATCH, int PART>
 __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg C) {
   // the mesh of this block: the context's, or in a batch the block's own
   // (its blocks [blk0, blk0 + nblk), elements [el0, el1))
@@ -1094,6 +1093,329 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
 
 template <int BS>
 constexpr int getdt_elements_per_block() { return BS - 2; }
+#else
+// Two kernels.  k_edge computes every edge of the mesh once
+// (bl_setup.cuh: its slots); k_getdt then takes each element's four edges
+// and does what depends on the element.  The edge viscosity's limiter, edge
+// coefficient and lengths are the same seen from either element of an edge;
+// one kernel per element computed each twice, a thread's four faces one
+// after another.  Sedov 512x512: 145 us in one kernel, 69.6 us in two (218
+// FP64 instructions, 31 divides and 9 square roots an element against about
+// 110, 7 and 4); a 16,000-element Sod tube, where the one-thread chain was
+// all of it, 42 to 28 us.
+// the limiter of two ratios (hydro_kn_edgeviscosity.f90:185-199)
+__device__ __forceinline__ double limit2(double r1, double r2) {
+  return maxF(0.0, minF(minF(minF(half(r1 + r2), twice(r1)), twice(r2)), 1.0));
+}
+
+// the codes of an edge's continuing faces (bl_setup.cuh)
+constexpr int kEndMirror = -2, kEndAdjacent = -3;
+
+// position and velocity differences along a face, or a wall's ratio
+struct EndD {
+  double dx, dy, du, dv;
+};
+__device__ __forceinline__ EndD node_diff(const DevFields& F, int a, int b) {
+  EndD d;
+  d.dx = F.ndx[b] - F.ndx[a];
+  d.dy = F.ndy[b] - F.ndy[a];
+  d.du = F.ndu[b] - F.ndu[a];
+  d.dv = F.ndv[b] - F.ndv[a];
+  return d;
+}
+
+// biased exponent of |x| within [1023 + lo, 1023 + hi]
+__device__ __forceinline__ bool exp_in(double x, int lo, int hi) {
+  const int e = (int)((unsigned long long)bits64(x) >> 52) & 0x7ff;
+  return (unsigned)(e - (1023 + lo)) <= (unsigned)(hi - lo);
+}
+// The limiter as the reference forms it, with its cut-offs: unit vectors
+// and one quotient per ratio.  Out of line: k_edge needs it only for
+// operands outside the range its own form covers.
+static __device__ __noinline__ double limiter_general(double du, double dv, double dx, double dy,
+                                                      int c1, EndD d1, int c2, EndD d2, double zc) {
+  const FaceQ f = face_q(du, dv, dx, dy, zc);
+  const double r1 = c1 < 0 && c1 != kEndAdjacent ? (c1 == kEndMirror ? 1.0 : 0.0)
+                                                 : nb_ratio(f, d1.dx, d1.dy, d1.du, d1.dv, zc);
+  const double r2 = c2 < 0 && c2 != kEndAdjacent ? (c2 == kEndMirror ? 1.0 : 0.0)
+                                                 : nb_ratio(f, d2.dx, d2.dy, d2.du, d2.dv, zc);
+  return limit2(r1, r2);
+}
+
+// ================================================================ k_edge
+
+// One thread per slot; a block of BS threads takes BS - 2 consecutive
+// slots, its first and last threads hold the neighbours of those and only
+// publish.  Every thread publishes its edge's differences; an edge takes a
+// continuing face from the thread beside it where the table says that it is
+// that slot's edge (on meshes numbered along mesh lines all but the walls
+// and the irregular faces), and gathers it from the nodes otherwise.
+//
+// With D = (dx, dy) and U = (du, dv) of this edge and
+// D', U' of a continuing one, the reference's ratio is, in real arithmetic
+// and away from its cut-offs, r = (U'.U |D|^2) / (|U|^2 D'.D): no square
+// root, no unit vector.  The two products U'.U and D'.D are the same for
+// the neighbour that continues into this edge, so each thread forms those
+// with the next slot and hands them on: four operations a slot for both
+// ends.  The limiter max(0, min((r1 + r2)/2, 2 r1, 2 r2, 1)) is then one
+// quotient over the common denominator, and none where it is 0 or 1.  It
+// holds while the squares and products keep clear of the range's ends and
+// of zerocut (tested on their exponents: lengths from 2^-40 to 2^40,
+// velocity differences from 2^-80 to 2^80, zerocut at most 2^-132; the
+// default is 1e-40); other operands take limiter_general.  An edge whose
+// velocity difference is at most zerocut gives no viscosity and skips the
+// rest, as whole warps of still fluid do.
+// Per edge it leaves (du, dv, E, EL), E = edge coefficient / |U| (0 where
+// the reference cuts the edge) and EL = edge coefficient * |U|, and |D|^2.
+#ifndef BL_EDGE_MINB
+#define BL_EDGE_MINB 8
+#endif
+template <int BS, bool BATCH>
+__global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C) {
+  const int t = threadIdx.x;
+  const int slot = (int)blockIdx.x * (BS - 2) + t - 1;
+  bool in = slot >= 0 && slot < F.nslot;
+  if (!BATCH && (halted(F.step) || F.step->stop_next)) return;
+  int4 n = make_int4(0, 0, 0, 0), q = make_int4(-1, -1, -1, -1);
+  if (in) {
+    n = __ldg(F.es_n + slot);
+    q = __ldg(F.es_q + slot);
+    if (BATCH) {
+      const DevStep* S = el_step<true>(F, n.z);
+      in = !(halted(S) || S->stop_next);
+    }
+  }
+  __shared__ double s_d[4][BS];
+  EndD d = {0.0, 0.0, 0.0, 0.0};
+  if (in) d = node_diff(F, n.x, n.y);
+  s_d[0][t] = d.dx;
+  s_d[1][t] = d.dy;
+  s_d[2][t] = d.du;
+  s_d[3][t] = d.dv;
+  __syncthreads();
+  const double zc = C.zerocut;
+  auto diff = [&](int code, int node, int beside) {  // a continuing face's differences
+    EndD r;
+    if (code == kEndAdjacent) {
+      r.dx = s_d[0][beside];
+      r.dy = s_d[1][beside];
+      r.du = s_d[2][beside];
+      r.dv = s_d[3][beside];
+    } else {
+      r = node_diff(F, code, node);
+    }
+    return r;
+  };
+  __shared__ double s_p[BS], s_q[BS];
+  if (t < BS - 1) {
+    s_p[t] = fma(d.dv, s_d[3][t + 1], d.du * s_d[2][t + 1]);
+    s_q[t] = fma(d.dy, s_d[1][t + 1], d.dx * s_d[0][t + 1]);
+  }
+  __syncthreads();
+  if (!(in && t > 0 && t < BS - 1)) return;
+  const double squ = fma(d.dv, d.dv, d.du * d.du), sqx = fma(d.dy, d.dy, d.dx * d.dx);
+  double E = 0.0, EL = 0.0;
+  const double lu = SQRT(squ);
+  if (!C.ztq && !le_nn(lu, zc)) {
+    const double cs = SQRT(half(F.cs2[n.z] + F.cs2[n.w]));
+    auto dots = [&](int code, int node, int beside, double& P, double& Q) {
+      if (code == kEndAdjacent) {
+        const int k = beside < t ? beside : t;
+        P = s_p[k];
+        Q = s_q[k];
+      } else if (code < 0) {  // a wall's ratio 0, a mirrored face's 1
+        P = code == kEndMirror ? squ : 0.0;
+        Q = sqx;
+      } else {
+        const EndD o = node_diff(F, code, node);
+        P = fma(d.dv, o.dv, d.du * o.du);
+        Q = fma(d.dy, o.dy, d.dx * o.dx);
+      }
+    };
+    double P1, Q1, P2, Q2, lim;
+    dots(q.x, q.y, t - 1, P1, Q1);
+    dots(q.z, q.w, t + 1, P2, Q2);
+    bool cut = false;
+    if (zc <= 0x1p-132 && exp_in(squ, -160, 160) && exp_in(sqx, -80, 80) &&
+        exp_in(Q1, -80, 80) && exp_in(Q2, -80, 80) && exp_in(P1, -1023, 300) &&
+        exp_in(P2, -1023, 300)) {
+      const double QQ = Q1 * Q2;
+      const double S1 = xorsign(P1 * Q2, QQ), S2 = xorsign(P2 * Q1, QQ);
+      const double m = minF(minF(half(S1 + S2), twice(S1)), twice(S2));
+      const double num = m * sqx, den = absF(QQ) * squ;
+      lim = gtF(num, 0.0) ? (gtF(den, num) ? DIV(num, den) : 1.0) : 0.0;
+    } else {
+      const EndD none = {0.0, 0.0, 0.0, 0.0};
+      const EndD o1 = q.x >= 0 || q.x == kEndAdjacent ? diff(q.x, q.y, t - 1) : none;
+      const EndD o2 = q.z >= 0 || q.z == kEndAdjacent ? diff(q.z, q.w, t + 1) : none;
+      lim = limiter_general(d.du, d.dv, d.dx, d.dy, q.x, o1, q.z, o2, zc);
+      cut = le_nn(SQRT(sqx), zc);
+    }
+    const double edv = half(1.0 - lim) *
+                       ((F.rho[n.z] + F.rho[n.w]) * fma(C.cvisc2, lu, C.cvisc1 * cs));
+    EL = edv * lu;
+    E = cut ? 0.0 : DIV(edv, lu);
+  }
+  F.erec[slot] = make_d4(d.du, d.dv, E, EL);
+  F.esqx[slot] = sqx;
+}
+
+// ================================================================ k_getdt
+
+// The element's CFL candidate over its squared signal speed cs2v, and its
+// divergence candidate, from its coefficients and its edges' velocity
+// differences and squared lengths (exact in real arithmetic):
+// - with T1 = a1 b2 - a2 b1, T3 = a3 b2 - a2 b3 and the quarter volume
+//   cross = a1 b3 - a3 b1, half the cross product of face f with the vector
+//   from its midpoint to the centroid is W = cross + T3, cross + T1,
+//   cross - T3, cross - T1; the reference's squared distance over squared
+//   length of the side across face f (geometry_kn_dln) is 16 W^2 / |D|^2;
+// - sum u_j (coefficient) is b1 (du3 - du1) + b3 (du0 - du2)
+//   - a1 (dv3 - dv1) - a3 (dv0 - dv2).
+__device__ __forceinline__ double cfl_candidate(const DevFields& F, const DevCfg& C, int iel,
+                                                const double* W, const double* sq, double a1,
+                                                double a2, double a3, double b1, double b2,
+                                                double b3, double cs2v) {
+  const int ireg = __ldg(F.ielreg + iel);
+  if (__ldg(C.zdtnotreg + ireg)) return DBL_MAX;
+  if (__ldg(C.zmidlength + ireg)) {  // min over sides of |midpoint difference|^2
+    const double r0 = a3 * a3 + b3 * b3, r1 = a1 * a1 + b1 * b1;
+    return DIV(times4(minF_nn(r0, r1)), cs2v);
+  }
+  bool plain = true;
+#pragma unroll
+  for (int f = 0; f < 4; f++) plain = plain && !gt_nn(C.zcut, sq[f]) && exp_in(sq[f], -160, 160);
+  if (plain) {
+    // the smallest quotient by cross-multiplication: two products in place
+    // of a divide
+    double n = W[0] * W[0], d = sq[0];
+#pragma unroll
+    for (int f = 1; f < 4; f++) {
+      const double nf = W[f] * W[f];
+      if (gt_nn(n * sq[f], nf * d)) {
+        n = nf;
+        d = sq[f];
+      }
+    }
+    return DIV(ldexpF<4>(n), d * cs2v);
+  }
+  // a face shorter than sqrt(zcut) counts with the distance from the
+  // opposite midpoint to its first corner
+  const double cx[4] = {a3, -a1, -a3, a1}, cy[4] = {b3, -b1, -b3, b1};
+  const double hx[4] = {a1 - a2, a2 + a3, -(a1 + a2), a2 - a3};
+  const double hy[4] = {b1 - b2, b2 + b3, -(b1 + b2), b2 - b3};
+  double m = HUGE_VAL;
+#pragma unroll
+  for (int f = 0; f < 4; f++) {
+    double r;
+    if (gt_nn(C.zcut, sq[f])) {
+      const double x = twice(cx[f]) + hx[f], y = twice(cy[f]) + hy[f];
+      r = x * x + y * y;
+    } else {
+      r = DIV(ldexpF<4>(W[f] * W[f]), sq[f]);
+    }
+    m = minF_nn(m, r);
+  }
+  return DIV(m, cs2v);
+}
+
+// One thread per element: its corner viscosity forces and viscosity from
+// its edges, elcs2 + elvisc, and its CFL and divergence candidates; then
+// the dt reduction.
+template <int BS, bool BATCH>
+__global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg C) {
+  // the mesh of this block: the context's, or in a batch the block's own
+  // (its blocks [blk0, blk0 + nblk), elements [el0, el1))
+  DevStep* S = F.step;
+  int blk0 = 0, nblk = (int)gridDim.x, el0 = 0, el1 = F.nel;
+  const DevInst* I = nullptr;
+  if (BATCH) {
+    const int m = __ldg(F.blkinst + blockIdx.x);
+    I = F.inst + m;
+    S = F.steps + m;
+    blk0 = I->blk_begin;
+    nblk = I->blk_end - I->blk_begin;
+    el0 = I->el_begin;
+    el1 = I->el_end;
+  }
+  if (halted(S)) return;
+  if (S->stop_next) {            // bl_run: the previous step reached time_end
+    if ((int)blockIdx.x == blk0 && threadIdx.x == 0) S->halted = 1;
+    return;
+  }
+  const int iel = el0 + ((int)blockIdx.x - blk0) * BS + (int)threadIdx.x;
+  double cflv = HUGE_VAL;        // sentinel above HUGE(1.0)
+  int cfli = 0x7fffffff;
+  double divv = DBL_MIN;         // TINY(1.0)
+  int divi = -1;
+  if (iel < el1) {
+    const uint4 er4 = __ldg(F.eref + iel);
+    const unsigned er[4] = {er4.x, er4.y, er4.z, er4.w};
+    double visc = 0.0;
+    double du[4], dv[4], sq[4], W[4], edx[4], edy[4];
+    const double a1 = F.a1[iel], a2 = F.a2[iel], a3 = F.a3[iel];
+    const double b1 = F.b1[iel], b2 = F.b2[iel], b3 = F.b3[iel];
+    const double vol = F.vol[iel];
+    {
+      const double cross = quarter(vol);
+      const double t1 = a1 * b2 - a2 * b1, t3 = a3 * b2 - a2 * b3;
+      W[0] = cross + t3;
+      W[1] = cross + t1;
+      W[2] = cross - t3;
+      W[3] = cross - t1;
+    }
+    const double zc = C.zerocut;
+    // |midpoint to centroid| above zerocut: (a3,b3) for faces 0 and 2,
+    // (a1,b1) for 1 and 3 (a component above it says so without the square)
+    const bool cut0 = !(gt_nn(absF(a3), zc) || gt_nn(absF(b3), zc)) && le_nn(a3 * a3 + b3 * b3, zc * zc);
+    const bool cut1 = !(gt_nn(absF(a1), zc) || gt_nn(absF(b1), zc)) && le_nn(a1 * a1 + b1 * b1, zc * zc);
+    double vmax = 0.0;
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+      const unsigned slot = er[f] >> 1;
+      const d4 R = F.erec[slot];
+      sq[f] = F.esqx[slot];
+      const double sg = from_bits64((long long)((unsigned long long)(er[f] & 1u) << 63));
+      du[f] = xorsign(R.x, sg);
+      dv[f] = xorsign(R.y, sg);
+      vmax = maxF_nn(vmax, R.w);  // never negative
+      // edge force (hydro_kn_edgeviscosity.f90:219-282): the reference
+      // normalises the midpoint-to-centroid vector c, orients it by the
+      // sign of its product with the face vector (that of W) and scales it
+      // back by |c|; so the force is U E times -+(U x c)
+      const double cx = (f & 1) ? a1 : a3, cy = (f & 1) ? b1 : b3;
+      const double g = dv[f] * cx - du[f] * cy;  // c has the other sign for faces 1 and 2
+      const double w6 = (f == 1 || f == 2) ? negxorsign(g, W[f]) : xorsign(g, W[f]);
+      const double d = R.z * w6;
+      const bool cut = geF(zc, w6) || ((f & 1) ? cut1 : cut0);
+      edx[f] = cut ? 0.0 : du[f] * d;
+      edy[f] = cut ? 0.0 : dv[f] * d;
+    }
+    if (!C.ztq) {
+      visc = DIV(twice(vmax), maxF(F.rho[iel], zc));
+      F.cnviscx[iel] = make_d4(edx[0] - edx[3], edx[1] - edx[0], edx[2] - edx[1], edx[3] - edx[2]);
+      F.cnviscy[iel] = make_d4(edy[0] - edy[3], edy[1] - edy[0], edy[2] - edy[1], edy[3] - edy[2]);
+      F.visc[iel] = visc;
+    } else {
+      visc = F.visc[iel];
+    }
+    const double cs2v = signal_speed(F, iel, visc);
+    cflv = cfl_candidate(F, C, iel, W, sq, a1, a2, a3, b1, b2, b3, cs2v);
+    cfli = iel;
+    const double w = b1 * (du[3] - du[1]) + b3 * (du[0] - du[2]) - a1 * (dv[3] - dv[1]) -
+                     a3 * (dv[0] - dv[2]);
+    const double dd = DIV(absF(w), vol);
+    if (gt_nn(dd, divv)) {
+      divv = dd;
+      divi = iel;
+    }
+  }
+  getdt_finish<BS, BATCH>(F, C, S, cflv, cfli, divv, divi, blk0, nblk, el0, I);
+}
+
+template <int BS>
+constexpr int getdt_elements_per_block() { return BS; }
+#endif
 #else
 
 template <int BS, bool BATCH, class L = DevLayout>
@@ -1673,6 +1995,7 @@ __global__ void __launch_bounds__(32 * kClosureWarps) k_mix_closure(DevFields F,
 
 static constexpr int BS_DT = 128;
 static constexpr int BS_EL = 128;
+static constexpr int BS_ED = 128;  // k_edge
 static constexpr int BS_ND = 256;
 
 // one block per getdt_elements_per_block elements
@@ -1686,19 +2009,25 @@ int getdt_blocks(int nel) {
 // spread of finishing times is a spread of their speeds, not of their work)
 int getdt_grid(int nel) { return getdt_blocks(nel); }
 
+// k_edge: BS_ED - 2 slots a block
+[[maybe_unused]] static int edge_grid(int nslot) { return (nslot + BS_ED - 3) / (BS_ED - 2); }
+
 int getdt_launches(const DevCfg& C) {
-#if BL_FAST_ALGEBRA && BL_GETDT_SPLIT
+#if BL_MIXED
   return C.ztq ? 1 : 2;
 #else
   (void)C;
-  return 1;
+  return BL_FAST_ALGEBRA ? 2 : 1;
 #endif
 }
 void launch_getdt(const DevFields& F, const DevCfg& C, cudaStream_t s) {
-#if BL_FAST_ALGEBRA && BL_GETDT_SPLIT
+#if BL_MIXED
   if (!C.ztq) k_getdt<BS_DT, false, 1><<<getdt_grid(F.nel), BS_DT, 0, s>>>(F, C);
   k_getdt<BS_DT, false, 2><<<getdt_grid(F.nel), BS_DT, 0, s>>>(F, C);
 #else
+#if BL_FAST_ALGEBRA
+  k_edge<BS_ED, false><<<edge_grid(F.nslot), BS_ED, 0, s>>>(F, C);
+#endif
   k_getdt<BS_DT, false><<<getdt_grid(F.nel), BS_DT, 0, s>>>(F, C);
 #endif
 }
@@ -1733,10 +2062,13 @@ void launch_mix_closure_batch(const DevFields& F, const DevCfg& C, cudaStream_t 
 // a batch of meshes: k_getdt over each mesh's own blocks, the rest over all
 // elements or nodes, each reading the step header of its mesh
 void launch_getdt_batch(const DevFields& F, const DevCfg& C, cudaStream_t s) {
-#if BL_FAST_ALGEBRA && BL_GETDT_SPLIT
+#if BL_MIXED
   if (!C.ztq) k_getdt<BS_DT, true, 1><<<F.nblk_batch, BS_DT, 0, s>>>(F, C);
   k_getdt<BS_DT, true, 2><<<F.nblk_batch, BS_DT, 0, s>>>(F, C);
 #else
+#if BL_FAST_ALGEBRA
+  k_edge<BS_ED, true><<<edge_grid(F.nslot), BS_ED, 0, s>>>(F, C);
+#endif
   k_getdt<BS_DT, true><<<F.nblk_batch, BS_DT, 0, s>>>(F, C);
 #endif
 }
