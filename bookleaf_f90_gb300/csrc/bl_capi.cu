@@ -554,6 +554,7 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
   up(x, F.b1, dh[BL_B1], nel);
   up(x, F.b2, dh[BL_B2], nel);
   up(x, F.b3, dh[BL_B3], nel);
+  F.geom_x = !(dh[BL_A2] && dh[BL_B2]);
   up(x, F.cnwt, dh[BL_CNWT], nel);
   up(x, F.cnmass, dh[BL_CNMASS], nel);
   up(x, F.cnviscx, dh[BL_CNVISCX], nel);
@@ -1144,15 +1145,20 @@ int bl_sync_to_host(bl_ctx* x, int id) {
   return BL_SUCCESS;
 }
 
-int bl_sync_to_device(bl_ctx* x, int id) {
-  if (!x) return BL_FAILURE;
-  if (id == 0) {
-    for (int k : kStateIds) {
-      int rc = bl_sync_to_device(x, k);
-      if (rc != BL_SUCCESS) return rc;
-    }
-    return BL_SUCCESS;
-  }
+// Whether the kernels may take the element coefficients a1..b3 for those of
+// the node positions (DevFields::geom_x = 0): they are after a whole upload,
+// not when either was uploaded on its own.  The device loops' graphs hold
+// the flag as it was at their capture.
+static void set_geom_x(bl_ctx* x, int v) {
+  if (x->F.geom_x == v) return;
+  x->F.geom_x = v;
+  if (x->gexec) cudaGraphExecDestroy(x->gexec);
+  x->gexec = nullptr;
+  if (x->bexec) cudaGraphExecDestroy(x->bexec);
+  x->bexec = nullptr;
+}
+
+static int upload_field(bl_ctx* x, int id) {
   if (id < 1 || id > BL_NID || !x->host[id]) return BL_SUCCESS;
   int kind;
   size_t n = field_count(x, id, kind);
@@ -1164,6 +1170,20 @@ int bl_sync_to_device(bl_ctx* x, int id) {
     r = cudaMemcpy(x->cs2_is_v ? x->F.cs2 : x->F.cs2v, x->host[id], n * sizeof(double),
                    cudaMemcpyHostToDevice);
   return r == cudaSuccess ? BL_SUCCESS : BL_FAILURE;
+}
+
+int bl_sync_to_device(bl_ctx* x, int id) {
+  if (!x) return BL_FAILURE;
+  if (id == 0) {
+    for (int k : kStateIds) {
+      int rc = upload_field(x, k);
+      if (rc != BL_SUCCESS) return rc;
+    }
+    set_geom_x(x, !(x->host[BL_A2] && x->host[BL_B2]));
+    return BL_SUCCESS;
+  }
+  if (id == BL_NDX || id == BL_NDY || (id >= BL_A1 && id <= BL_B3)) set_geom_x(x, 1);
+  return upload_field(x, id);
 }
 
 int bl_synchronize(bl_ctx* x) {

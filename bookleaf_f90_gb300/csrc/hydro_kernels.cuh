@@ -169,16 +169,7 @@ struct Iso {
 // corner weights, (3b3 -+ b2)(3a1 -+ a2) - (3a3 -+ a2)(3b1 -+ b2) over 9,
 // gives cross + (T3 - T1)/3, cross + (T1 + T3)/3, cross - (T3 - T1)/3,
 // cross - (T1 + T3)/3 for corners 0..3 (exact in real arithmetic).
-__device__ __forceinline__ Iso getiso(const double* x, const double* y) {
-  Iso g;
-  const double ux = x[2] - x[0], vx = x[1] - x[3];
-  const double uy = y[2] - y[0], vy = y[1] - y[3];
-  g.a1 = quarter(ux + vx);
-  g.a3 = quarter(ux - vx);
-  g.a2 = quarter((x[0] + x[2]) - (x[1] + x[3]));
-  g.b1 = quarter(uy + vy);
-  g.b3 = quarter(uy - vy);
-  g.b2 = quarter((y[0] + y[2]) - (y[1] + y[3]));
+__device__ __forceinline__ void iso_volumes(Iso& g) {
   g.cross = g.a1 * g.b3 - g.a3 * g.b1;
   const double t1 = g.a1 * g.b2 - g.a2 * g.b1;
   const double t3 = g.a3 * g.b2 - g.a2 * g.b3;
@@ -190,6 +181,18 @@ __device__ __forceinline__ Iso getiso(const double* x, const double* y) {
   g.w2 = fma(-g.td, o3, g.cross);
   g.w3 = fma(-g.ts, o3, g.cross);
   g.vol = times4(g.cross);
+}
+__device__ __forceinline__ Iso getiso(const double* x, const double* y) {
+  Iso g;
+  const double ux = x[2] - x[0], vx = x[1] - x[3];
+  const double uy = y[2] - y[0], vy = y[1] - y[3];
+  g.a1 = quarter(ux + vx);
+  g.a3 = quarter(ux - vx);
+  g.a2 = quarter((x[0] + x[2]) - (x[1] + x[3]));
+  g.b1 = quarter(uy + vy);
+  g.b3 = quarter(uy - vy);
+  g.b2 = quarter((y[0] + y[2]) - (y[1] + y[3]));
+  iso_volumes(g);
   return g;
 }
 #else
@@ -347,63 +350,7 @@ __device__ __forceinline__ void force_pq(double p, double a1, double a3, double 
 #endif
 }
 
-#if BL_FAST_ALGEBRA
-// Fast build: hydro_kn_getforceSP (hydro_kn_getforce.f90:109-188) from the
-// element's iso-parametric coefficients.  With the corners written as
-// s - a1 + a2 - a3, s + a1 - a2 - a3, s + a1 + a2 + a3, s - a1 - a2 + a3
-// (s the centroid), the sub-quad of corner j (the corner, the edge midpoint
-// after it, the centroid, the edge midpoint before it) has the x
-// coefficients (w3, w4) = (P, Q), (R, -P), (-S, -R), (-Q, S), all over 4,
-// with P = 2a1 - a2, Q = 2a3 - a2, R = 2a3 + a2, S = 2a1 + a2, and the y
-// coefficients (w5, w6) likewise from the b's.  Expanding (all exact in
-// real arithmetic):
-// - the sub-volumes 4(w3 w6 - w4 w5) are V_j = cross + td/2, cross + ts/2,
-//   cross - td/2, cross - ts/2 (cross = a1 b3 - a3 b1, ts = T1 + T3,
-//   td = T3 - T1, T1 = a1 b2 - a2 b1, T3 = a3 b2 - a2 b3);
-// - with p_j = cs2 (spmass_j / V_j - rho), the reference's corner x forces
-//   lfx(j,1) = p_j (w5 - w6) and lfx(j,2) = p_j (w5 + w6) are p_j c_j / 2
-//   and p_j C_j / 2 with c = (db, sb, -db, -sb) and
-//   C = (sb - b2, b2 - db, -(sb + b2), db + b2), db = b1 - b3, sb = b1 + b3;
-//   lfx(j,3) and lfx(j,4) are their negatives;
-// - in the reference's gather of the sub-quad forces to the corners the
-//   midpoint terms of adjacent sub-quads cancel pairwise, leaving, with
-//   M_j = p_j C_j and G = db (p0 - p2) + sb (p1 - p3),
-//   fx0 += w1/8 (4 p0 db + 2 (M3 - M1) - G),
-//   fx1 += w1/8 (4 p1 sb + 2 (M0 - M2) - G),
-//   fx2 -= w1/8 (4 p2 db + 2 (M3 - M1) + G),
-//   fx3 -= w1/8 (4 p3 sb + 2 (M0 - M2) + G);
-// - the y forces are the same with the a's in place of the b's and the
-//   sign of w1 reversed.
-__device__ __forceinline__ void sp_direction(double k, const double* p, double e02, double e13,
-                                             double c1, double c2, double c3, double* f) {
-  const double dd = c1 - c3, ss = c1 + c3;
-  const double m0 = p[0] * (ss - c2), m1 = p[1] * (c2 - dd);
-  const double m2 = -(p[2] * (ss + c2)), m3 = p[3] * (dd + c2);
-  const double d13 = twice(m3 - m1), d02 = twice(m0 - m2);
-  const double g = fma(dd, e02, ss * e13);
-  const double d4 = times4(dd), s4 = times4(ss);
-  f[0] = fma(k, fma(p[0], d4, d13) - g, f[0]);
-  f[1] = fma(k, fma(p[1], s4, d02) - g, f[1]);
-  f[2] = fma(-k, fma(p[2], d4, d13) + g, f[2]);
-  f[3] = fma(-k, fma(p[3], s4, d02) + g, f[3]);
-}
-
-__device__ __forceinline__ void force_sp_iso(double w1, double rho, double cs2, double cross,
-                                             double ts, double td, double a1, double a2,
-                                             double a3, double b1, double b2, double b3,
-                                             const d4& spm, double* fx, double* fy) {
-  const double V[4] = {fma(td, 0.5, cross), fma(ts, 0.5, cross), fma(-td, 0.5, cross),
-                       fma(-ts, 0.5, cross)};
-  const double cr = cs2 * rho;
-  double p[4];
-#pragma unroll
-  for (int j = 0; j < 4; j++) p[j] = fma(cs2, DIV(c4(spm, j), V[j]), -cr);
-  const double e02 = p[0] - p[2], e13 = p[1] - p[3];
-  const double k = ldexpF<-3>(w1);
-  sp_direction(k, p, e02, e13, b1, b2, b3, fx);
-  sp_direction(-k, p, e02, e13, a1, a2, a3, fy);
-}
-#else
+#if !BL_FAST_ALGEBRA
 // hydro_kn_getforceSP (hydro_kn_getforce.f90:109-188)
 __device__ void force_sp(double w1, double rho, double cs2, const double* cx, const double* cy,
                          const d4& spm, double* fx, double* fy) {
@@ -461,6 +408,7 @@ __device__ void force_sp(double w1, double rho, double cs2, const double* cx, co
 }
 #endif
 
+#if !BL_FAST_ALGEBRA
 // hydro_kn_getforceHG (hydro_kn_getforce.f90:73-107)
 __device__ __forceinline__ void force_hg(double kappa, double rho, double area, double rdt,
                                          const double* u, const double* v, double* fx,
@@ -479,6 +427,7 @@ __device__ __forceinline__ void force_hg(double kappa, double rho, double area, 
   fy[2] = fy[2] + w3;
   fy[3] = fy[3] - w3;
 }
+#endif
 
 // hydro_kn_getenergy (hydro_kn_getenergy.f90:29-52): the increment w1*dt
 __device__ __forceinline__ double energy_update(double e, double m, double zerocut, double dt,
@@ -1595,6 +1544,236 @@ constexpr int getdt_elements_per_block() { return BS; }
 
 // ================================================================ k_lag_force
 
+#if BL_FAST_ALGEBRA
+// Fast build.  Only the energy needs the predictor's forces, and only their
+// work sum f_j . u_j, so that is formed directly; the half-step geometry
+// follows from the element's own coefficients, which are linear in the
+// corner positions; the corrector's pressure, sub-zonal and hourglass forces
+// share their sums.  (All exact in real arithmetic.)  With
+//   d = (b1 - b3), s = (b1 + b3), U02 = u0 - u2, U13 = u1 - u3,
+//   h = u0 - u1 + u2 - u3 (and the same with a and v for y, sign reversed):
+// - pressure work: p Dv, Dv = d U02 + s U13 - (y);
+// - a1, a2, a3 at the half step: a1 + dt/8 (U13 - U02), a2 + dt/8 h,
+//   a3 - dt/8 (U02 + U13);
+// - sub-zonal pressures (hydro_kn_getforce.f90:109-188): the sub-quad of
+//   corner j has the volume V_j = cross + td/2, cross + ts/2, cross - td/2,
+//   cross - ts/2 (cross = a1 b3 - a3 b1, ts = T1 + T3, td = T3 - T1,
+//   T1 = a1 b2 - a2 b1, T3 = a3 b2 - a2 b3) and the pressure p_j = cs2
+//   (spmass_j / V_j - rho); in the reference's gather of the sub-quads'
+//   forces to the corners the midpoint terms of adjacent ones cancel
+//   pairwise.  With P_j = pmerit p_j / 2, S02 = P0 + P2, M02 = P0 - P2 (S13,
+//   M13 likewise), the corner x forces are
+//     f0 =  d P0 + D13 - G, f2 = -d P2 - D13 - G,
+//     f1 =  s P1 + D02 - G, f3 = -s P3 - D02 - G,
+//     D13 = (d S13 - b2 M13)/2, D02 = (s S02 - b2 M02)/2,
+//     G = (d M02 + s M13)/4,
+//   and their work, with q_j = spmass_j / V_j,
+//     pmerit cs2 / 8 (2 Dv (sum q_j - 4 rho) + B (q0 - q2) - C (q1 - q3)),
+//     B = d h - 2 b2 U13 - (y), C = s h + 2 b2 U02 - (y).
+// 140 FP64 instructions an element with all forces on where the reference's
+// terms one by one took 206, and no corner positions gathered: Sedov
+// 512x512 108 -> 90 us (FP64 pipe 79 % busy over the SMs' active cycles, the
+// divide chains' latency the rest; 3, 5 and 6 blocks per SM and blocks of 64
+// and 256 threads are slower or equal), 42 -> 39 us at 90,000 elements.
+// Where the coefficients may not be those of the positions (F.geom_x: a2 or
+// b2 not registered, or positions uploaded on their own) the half-step
+// geometry is formed from the corners.
+struct SubZone {
+  double q[4];  // sub-zonal densities spmass_j / V_j
+};
+__device__ __forceinline__ SubZone sub_zone(double cross, double ts, double td, const d4& spm) {
+  SubZone z;
+  z.q[0] = DIV(spm.x, fma(td, 0.5, cross));
+  z.q[1] = DIV(spm.y, fma(ts, 0.5, cross));
+  z.q[2] = DIV(spm.z, fma(-td, 0.5, cross));
+  z.q[3] = DIV(spm.w, fma(-ts, 0.5, cross));
+  return z;
+}
+// one direction's corner forces (sg = 1: x from the b's, -1: y from the
+// a's); w the hourglass force of the even corners
+template <int SG>
+__device__ __forceinline__ void corner_forces(double d, double s, double c2, const double* P,
+                                              double S02, double M02, double S13, double M13,
+                                              double w, const d4& q, double* f) {
+  const double G = quarter(fma(d, M02, s * M13));
+  const double D13 = half(fma(d, S13, -(c2 * M13))), D02 = half(fma(s, S02, -(c2 * M02)));
+  if (SG > 0) {
+    const double e = w - G, o = -w - G;
+    f[0] = fma(d, P[0], (e + D13) + q.x);
+    f[1] = fma(s, P[1], (o + D02) + q.y);
+    f[2] = fma(-d, P[2], (e - D13) + q.z);
+    f[3] = fma(-s, P[3], (o - D02) + q.w);
+  } else {
+    const double e = w + G, o = G - w;
+    f[0] = fma(-d, P[0], (e - D13) + q.x);
+    f[1] = fma(-s, P[1], (o - D02) + q.y);
+    f[2] = fma(d, P[2], (e + D13) + q.z);
+    f[3] = fma(s, P[3], (o + D02) + q.w);
+  }
+}
+
+template <int BS, bool BATCH>
+__global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, DevCfg C) {
+  const int iel = blockIdx.x * BS + threadIdx.x;
+  if (iel >= F.nel) return;
+  DevStep* S = el_step<BATCH>(F, iel);
+  if (halted(S)) return;
+  const double dt = S->dt;
+  const double hdt = half(dt);   // time_dr_setpredictor dts / getvertex step
+  const double zc = C.zerocut;
+  const int4 nd = __ldg(F.ielnd + iel);
+  const int n[4] = {nd.x, nd.y, nd.z, nd.w};
+  double u[4], v[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    u[j] = F.ndu[n[j]];
+    v[j] = F.ndv[n[j]];
+  }
+  const d4 qx = F.cnviscx[iel], qy = F.cnviscy[iel];
+  const int ireg = __ldg(F.ielreg + iel);
+  const int mat = __ldg(F.ielmat + iel);
+  const double m = F.mass[iel];
+  const double e0 = F.e[iel];
+  const int imx = F.elmx ? F.elmx[iel] : -1;
+  const double a1 = F.a1[iel], a2 = F.a2[iel], a3 = F.a3[iel];
+  const double b1 = F.b1[iel], b2 = F.b2[iel], b3 = F.b3[iel];
+  const double u02 = u[0] - u[2], u13 = u[1] - u[3], v02 = v[0] - v[2], v13 = v[1] - v[3];
+  const double hu = (u[0] + u[2]) - (u[1] + u[3]), hv = (v[0] + v[2]) - (v[1] + v[3]);
+  const double pm = C.zsp ? __ldg(C.pmeritreg + ireg) : 0.0;
+  // ---- the predictor forces' work at t^n (hydro_dr_getforce, zcorrector false)
+  double work;
+  {
+    const double d = b1 - b3, s = b1 + b3, dy = a1 - a3, sy = a1 + a3;
+    const double Dv = (d * u02 + s * u13) - (dy * v02 + sy * v13);
+    work = F.p[iel] * Dv + qx.x * u[0] + qy.x * v[0] + qx.y * u[1] + qy.y * v[1] + qx.z * u[2] +
+           qy.z * v[2] + qx.w * u[3] + qy.w * v[3];
+    if (C.zsp) {
+      const double t1 = a1 * b2 - a2 * b1, t3 = a3 * b2 - a2 * b3;
+      const SubZone z = sub_zone(quarter(F.vol[iel]), t1 + t3, t3 - t1, F.spmass[iel]);
+      const double b22 = twice(b2), a22 = twice(a2);
+      const double B = (d * hu - b22 * u13) - (dy * hv - a22 * v13);
+      const double D = (s * hu + b22 * u02) - (sy * hv + a22 * v02);
+      const double sum = fma(-4.0, F.rho[iel], (z.q[0] + z.q[2]) + (z.q[1] + z.q[3]));
+      const double w = fma(twice(Dv), sum, fma(B, z.q[0] - z.q[2], -(D * (z.q[1] - z.q[3]))));
+      work = fma(ldexpF<-3>(pm) * F.cs2v[iel], w, work);
+    }
+  }
+  // ---- geometry at the half step (geometry_kn_getvertex with 0.5*dt,
+  // geometry_dr_getgeometry), density
+  Iso g;
+  if (!F.geom_x) {
+    const double r = quarter(hdt);
+    g.a1 = fma(r, u13 - u02, a1);
+    g.a2 = fma(r, hu, a2);
+    g.a3 = fma(-r, u02 + u13, a3);
+    g.b1 = fma(r, v13 - v02, b1);
+    g.b2 = fma(r, hv, b2);
+    g.b3 = fma(-r, v02 + v13, b3);
+    iso_volumes(g);
+  } else {
+    double xh[4], yh[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      xh[j] = F.ndx[n[j]] + hdt * u[j];
+      yh[j] = F.ndy[n[j]] + hdt * v[j];
+    }
+    g = getiso(xh, yh);
+  }
+  if (gtF(0.0, g.vol)) atomicMax(&S->negvol_pred, iel + 1 - el_base<BATCH>(F, iel));
+  const double rho = DIV(m, g.vol);
+  // ---- energy (hydro_kn_getenergy with dts = dt/2) and EoS
+  const double eh = e0 - DIV(work, maxF(m, zc)) * hdt;
+  double ph, cs2h;
+  eos_pc(C, mat, rho, eh, ph, cs2h);
+  double fx[4], fy[4];
+  // ---- mixed cells: component state at the half step
+  if (imx >= 0) {
+    const int c0 = F.imxfcp[imx], nc = F.imxncp[imx];
+    double ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
+    for (int k = 0; k < nc; k++) {
+      const int icp = c0 + k;
+      const double fr = F.frvol[icp];
+      // predictor component force with the t^n component state
+      double cfx[4], cfy[4];
+      force_pq(F.cpp[icp], a1, a3, b1, b3, F.cpviscx[icp],
+               F.cpviscy[icp], cfx, cfy);
+      // component energy with cpu = frvolume*cnu (utils_kn_mxgathercnav)
+      double cu[4], cv[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        cu[j] = fr * u[j];
+        cv[j] = fr * v[j];
+      }
+      const double cpm = F.cpm[icp];
+      const double cpe = energy_update(F.cpe[icp], cpm, zc, hdt, cfx, cfy, cu, cv);
+      F.cpe[icp] = cpe;  // the reference does not restore component energy
+      const double cpv = times4(g.a1 * g.b3 - g.a3 * g.b1) * fr;
+      const double cpr = DIV(cpm, cpv);
+      double cpp, cpc;
+      eos_pc(C, __ldg(F.icpmat + icp), cpr, cpe, cpp, cpc);
+      // corrector component force at the half-step state
+      force_pq(cpp, g.a1, g.a3, g.b1, g.b3, F.cpviscx[icp], F.cpviscy[icp], cfx, cfy);
+      F.cpfx[icp] = make_d4(cfx[0], cfx[1], cfx[2], cfx[3]);
+      F.cpfy[icp] = make_d4(cfy[0], cfy[1], cfy[2], cfy[3]);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        ax[j] = ax[j] + fr * cfx[j];
+        ay[j] = ay[j] + fr * cfy[j];
+      }
+    }
+    // corrector element force: P+Q+SP+HG are overwritten by the average
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      fx[j] = ax[j];
+      fy[j] = ay[j];
+    }
+  } else {
+    // ---- corrector force at the half step (zcorrector true)
+    const double d = g.b1 - g.b3, s = g.b1 + g.b3, dy = g.a1 - g.a3, sy = g.a1 + g.a3;
+    double wx = 0.0, wy = 0.0;
+    if (C.zhg) {  // hydro_kn_getforceHG (hydro_kn_getforce.f90:73-107)
+      const double w = -__ldg(C.kappareg + ireg) * rho * g.vol * S->rdt;
+      wx = w * hu;
+      wy = w * hv;
+    }
+    if (C.zsp) {
+      const SubZone z = sub_zone(g.cross, g.ts, g.td, F.spmass[iel]);
+      const double c = half(pm) * cs2h, cr = c * rho;
+      double P[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) P[j] = fma(c, z.q[j], -cr);
+      const double S02 = P[0] + P[2], M02 = P[0] - P[2], S13 = P[1] + P[3], M13 = P[1] - P[3];
+#pragma unroll
+      for (int j = 0; j < 4; j++) P[j] = P[j] + ph;
+      corner_forces<1>(d, s, g.b2, P, S02, M02, S13, M13, wx, qx, fx);
+      corner_forces<-1>(dy, sy, g.a2, P, S02, M02, S13, M13, wy, qy, fy);
+    } else {
+      fx[0] = fma(ph, d, qx.x);
+      fx[1] = fma(ph, s, qx.y);
+      fx[2] = fma(-ph, d, qx.z);
+      fx[3] = fma(-ph, s, qx.w);
+      fy[0] = fma(-ph, dy, qy.x);
+      fy[1] = fma(-ph, sy, qy.y);
+      fy[2] = fma(ph, dy, qy.z);
+      fy[3] = fma(ph, sy, qy.w);
+      if (C.zhg) {
+        fx[0] += wx;
+        fx[1] -= wx;
+        fx[2] += wx;
+        fx[3] -= wx;
+        fy[0] += wy;
+        fy[1] -= wy;
+        fy[2] += wy;
+        fy[3] -= wy;
+      }
+    }
+  }
+  F.cnfx[iel] = make_d4(fx[0], fx[1], fx[2], fx[3]);
+  F.cnfy[iel] = make_d4(fy[0], fy[1], fy[2], fy[3]);
+  F.rho_h[iel] = rho;
+  F.cnwt_h[iel] = make_d4(g.w0, g.w1, g.w2, g.w3);
+}
+#else
 template <int BS, bool BATCH>
 __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, DevCfg C) {
   const int iel = blockIdx.x * BS + threadIdx.x;
@@ -1625,15 +1804,7 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
   const double a1 = F.a1[iel], a3 = F.a3[iel], b1 = F.b1[iel], b3 = F.b3[iel];
   force_pq(F.p[iel], a1, a3, b1, b3, qx, qy, fx, fy);
   if (C.zsp) {
-#if BL_FAST_ALGEBRA
-    const double a2 = F.a2[iel], b2 = F.b2[iel];
-    const double cross = a1 * b3 - a3 * b1;
-    const double t1 = a1 * b2 - a2 * b1, t3 = a3 * b2 - a2 * b3;
-    force_sp_iso(__ldg(C.pmeritreg + ireg), F.rho[iel], F.cs2v[iel], cross, t1 + t3, t3 - t1, a1,
-                 a2, a3, b1, b2, b3, F.spmass[iel], fx, fy);
-#else
     force_sp(__ldg(C.pmeritreg + ireg), F.rho[iel], F.cs2v[iel], x, y, F.spmass[iel], fx, fy);
-#endif
   }
   // ---- half-step vertices (geometry_kn_getvertex with 0.5*dt)
   double xh[4], yh[4];
@@ -1695,12 +1866,7 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
     // ---- corrector force at the half step (zcorrector true)
     force_pq(ph, g.a1, g.a3, g.b1, g.b3, qx, qy, fx, fy);
     if (C.zsp) {
-#if BL_FAST_ALGEBRA
-      force_sp_iso(__ldg(C.pmeritreg + ireg), rho, cs2h, g.cross, g.ts, g.td, g.a1, g.a2, g.a3,
-                   g.b1, g.b2, g.b3, F.spmass[iel], fx, fy);
-#else
       force_sp(__ldg(C.pmeritreg + ireg), rho, cs2h, xh, yh, F.spmass[iel], fx, fy);
-#endif
     }
     if (C.zhg) force_hg(__ldg(C.kappareg + ireg), rho, g.vol, S->rdt, u, v, fx, fy);
   }
@@ -1709,6 +1875,7 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
   F.rho_h[iel] = rho;
   F.cnwt_h[iel] = make_d4(g.w0, g.w1, g.w2, g.w3);
 }
+#endif
 
 // ================================================================ k_lag_accel
 
@@ -1996,7 +2163,7 @@ __global__ void __launch_bounds__(32 * kClosureWarps) k_mix_closure(DevFields F,
 static constexpr int BS_DT = 128;
 static constexpr int BS_EL = 128;
 static constexpr int BS_ED = 128;  // k_edge
-static constexpr int BS_ND = 256;
+static constexpr int BS_ND = 128;
 
 // one block per getdt_elements_per_block elements
 int getdt_blocks(int nel) {
