@@ -37,6 +37,9 @@ __device__ __forceinline__ bool ale_on(const DevCfg& C, const DevStep* S) {
   return geF(t, C.ale_mintime) && geF(C.ale_maxtime, t);  // the IEEE >= on the integer pipe
 }
 
+__device__ __forceinline__ int node_at(const int4& n, int j) {
+  return j == 0 ? n.x : (j == 1 ? n.y : (j == 2 ? n.z : n.w));
+}
 __device__ __forceinline__ double cget(const d4* a, int iel, int j) {
   return reinterpret_cast<const double*>(a + iel)[j];
 }
@@ -94,13 +97,73 @@ __device__ __forceinline__ double grad_f32(double A, double B, double mA, double
 }
 #endif
 
+#if BL_FAST_ALGEBRA && !BL_MIXED
+// -1, 0 or 1 for a * b below, near (within 2^-18) or above c * d, from the
+// leading 21 bits and the exponents, on the integer pipe; 0 also for zero,
+// subnormal, infinite and NaN operands.  Signs are ignored.
+__device__ __forceinline__ int order_products(double a, double b, double c, double d) {
+  const unsigned ha = (unsigned)(bits64(a) >> 32) & 0x7fffffffu;
+  const unsigned hb = (unsigned)(bits64(b) >> 32) & 0x7fffffffu;
+  const unsigned hc = (unsigned)(bits64(c) >> 32) & 0x7fffffffu;
+  const unsigned hd = (unsigned)(bits64(d) >> 32) & 0x7fffffffu;
+  const unsigned lo = 0x00100000u, n = 0x7fe00000u;  // a normal number: hi - lo < n
+  if (ha - lo >= n || hb - lo >= n || hc - lo >= n || hd - lo >= n) return 0;
+  const int e = (int)(ha >> 20) + (int)(hb >> 20) - (int)(hc >> 20) - (int)(hd >> 20);
+  if (e > 2 || e < -2) return e > 0 ? 1 : -1;
+  const unsigned long long p =
+      ((unsigned long long)((ha & 0xfffffu) | lo) * ((hb & 0xfffffu) | lo)) << (2 + e);
+  const unsigned long long q =
+      ((unsigned long long)((hc & 0xfffffu) | lo) * ((hd & 0xfffffu) | lo)) << 2;
+  const long long diff = (long long)(p - q), near = (long long)(q >> 18);
+  return diff > near ? 1 : (diff < -near ? -1 : 0);
+}
+#endif
+
+// The remap limiters' gradient from the differences A, B of the advected
+// variable towards the two neighbours and the masses (or volumes) mA, mB of
+// the two sides: zero unless A and B have the same sign, else
+// min(|w8|, |A| / mA, |B| / mB) with the sign of S, w8 = (A mB^2 + B mA^2) /
+// (mA mB (mA + mB)).
+// Fast build: for positive mA and mB, w8 is the mean of A / mA and B / mB
+// weighted by mB and mA, which lies between them, so the minimum is the
+// smaller of those two quotients, and which one that is shows in the
+// products A mB and B mA: one divide, no product in the FP64 pipe, where
+// the three candidates took three divides and seven operations.  (Two
+// divides when the products are too near to tell.)
+__device__ __forceinline__ double limited_slope(double A, double B, double mA, double mB,
+                                                double S) {
+#if BL_MIXED
+  return grad_f32(A, B, mA, mB, S);
+#else
+#if BL_FAST_ALGEBRA
+  if (prod_le0(A, B)) return 0.0;
+  if (bits64(mA) > 0 && bits64(mB) > 0) {
+    const int o = order_products(A, mB, B, mA);
+    const double q = DIV(absF(o > 0 ? B : A), o > 0 ? mB : mA);
+    return signF(o == 0 ? minF_nn(q, DIV(absF(B), mB)) : q, S);
+  }
+#endif
+  const double w8 = DIV(A * mB * mB + B * mA * mA, mA * mB * (mA + mB));
+  double grad = sign_of(minF(minF(absF(w8), DIV(absF(A), mA)), DIV(absF(B), mB)), S);
+  if (prod_le0(A, B)) grad = 0.0;
+  return grad;
+#endif
+}
+
 // The limited face flux of ale_kn_fluxelvl for the pair (i1, i2=i1+2),
 // returning (fcflux(i1), fcflux(i2)) (ale_kn_advectors.f90:48-78).
-__device__ __forceinline__ void elvl_pair(int iel, int i1, const int* nb, const int* fc,
+__device__ __forceinline__ void elvl_pair(int i1, const int* nb, const int* fc,
                                           const d4* cnbasis, const double* own_b,
                                           double r1, double r2, const double* elvar,
                                           double rv, double& o1, double& o2) {
   const int i2 = i1 + 2;
+#if BL_FAST_ALGEBRA && !BL_MIXED
+  // nothing leaves through either face (fluid at rest)
+  if (((unsigned long long)(bits64(r1) | bits64(r2)) << 1) == 0) {
+    o1 = o2 = 0.0;
+    return;
+  }
+#endif
   const int iel2 = nb[i2];
   int j2 = fc[i2];
   double r3 = own_b[i2] + own_b[(i2 + 1) & 3];
@@ -111,17 +174,19 @@ __device__ __forceinline__ void elvl_pair(int iel, int i1, const int* nb, const 
   double w6 = r4 + cget(cnbasis, iel1, j2) + cget(cnbasis, iel1, (j2 + 1) & 3);
   double w1 = rv - elvar[iel2];
   double w2 = elvar[iel1] - rv;
-#if BL_MIXED
-  const double grad = grad_f32(w1, w2, w5, w6, w2);
+  const double grad = limited_slope(w1, w2, w5, w6, w2);
+#if BL_FAST_ALGEBRA && !BL_MIXED
+  // flow through the pair leaves through one face; the other's flux is 0
+  const bool z1 = (bits64(r1) << 1) == 0, z2 = (bits64(r2) << 1) == 0;
+  const double r = z1 ? r2 : r1;
+  const double o = r * fma(z1 ? negF(grad) : grad, (z1 ? r4 : r3) - half(r), rv);
+  o1 = z1 ? 0.0 : o;
+  o2 = z1 ? o : 0.0;
+  if (!z1 && !z2) o2 = r2 * fma(negF(grad), r4 - half(r2), rv);
 #else
-  double w3 = absF(w1), w4 = absF(w2);
-  double w8 = DIV(w1 * w6 * w6 + w2 * w5 * w5, w5 * w6 * (w5 + w6));
-  double grad = sign_of(minF(minF(absF(w8), DIV(w3, w5)), DIV(w4, w6)), w2);
-  if (prod_le0(w1, w2)) grad = 0.0;
-#endif
   o1 = r1 * (rv + grad * (r3 - half(r1)));
   o2 = r2 * (rv - grad * (r4 - half(r2)));
-  (void)iel;
+#endif
 }
 
 // ================================================================ k_ale_flux
@@ -162,7 +227,7 @@ __global__ void __launch_bounds__(BS) k_ale_flux(DevFields F, DevCfg C) {
     y1[j] = y0[j] + dt * (-F.ndvbar[n[j]]);
   }
 #endif
-  double fv[4], fvn[4];
+  double fv[4];
 #pragma unroll
   for (int jj = 0; jj < 4; jj++) {
     const int jp = (jj + 1) & 3;
@@ -176,33 +241,19 @@ __global__ void __launch_bounds__(BS) k_ale_flux(DevFields F, DevCfg C) {
     double d = face_dv(x0[jj], x0[jp], y0[jj], y0[jp], x1[jp], x1[jj], y1[jp], y1[jj]);
 #endif
     fv[jj] = gtF(zc, d) ? 0.0 : d;
-    double dn = -d;   // the neighbour's volume of the same face
-    fvn[jj] = gtF(zc, dn) ? 0.0 : dn;
   }
   const int4 ee = __ldg(F.ielel + iel);
   const int nb[4] = {ee.x, ee.y, ee.z, ee.w};
   const int fcp = __ldg(F.ielfc + iel);
   const int fc[4] = {fc_of(fcp, 0), fc_of(fcp, 1), fc_of(fcp, 2), fc_of(fcp, 3)};
-  // ale_kn_sumflux(fcdv)
-  double totv = 0.0;
-#pragma unroll
-  for (int i1 = 0; i1 < 2; i1++) {
-    const int i2 = i1 + 2;
-    double w1 = fvn[i1], w2 = fvn[i2];
-    if (nb[i1] == iel) w1 = 0.0;
-    if (nb[i2] == iel) w2 = 0.0;
-    totv = totv - fv[i1] - fv[i2] + w1 + w2;
-  }
   // ale_kn_fluxelvl(cnwt, fcdv, eldensity)
   const d4 cw = F.cnwt[iel];
   const double ob[4] = {cw.x, cw.y, cw.z, cw.w};
   const double rv = F.rho[iel];
   double fm[4];
-  elvl_pair(iel, 0, nb, fc, F.cnwt, ob, fv[0], fv[2], F.rho, rv, fm[0], fm[2]);
-  elvl_pair(iel, 1, nb, fc, F.cnwt, ob, fv[1], fv[3], F.rho, rv, fm[1], fm[3]);
+  elvl_pair(0, nb, fc, F.cnwt, ob, fv[0], fv[2], F.rho, rv, fm[0], fm[2]);
+  elvl_pair(1, nb, fc, F.cnwt, ob, fv[1], fv[3], F.rho, rv, fm[1], fm[3]);
   F.fcdm[iel] = make_d4(fm[0], fm[1], fm[2], fm[3]);
-  F.fcdv[iel] = make_d4(fv[0], fv[1], fv[2], fv[3]);
-  F.cutm_el[iel] = totv;  // carried to k_ale_el
 }
 
 // ================================================================ k_ale_el
@@ -221,6 +272,20 @@ __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
   const d4 fm4 = F.fcdm[iel];
   const double fm[4] = {fm4.x, fm4.y, fm4.z, fm4.w};
   // ale_kn_sumflux(fcdm): neighbour's flux of the shared face
+  const double mpr = F.mass[iel];
+#if BL_FAST_ALGEBRA
+  // each face's net flux once: their sum is the element's gain (and four
+  // times each corner's, ale_kn_fluxbasisnd), the difference of opposite
+  // ones the corner mass-flux basis
+  double net[4];
+#pragma unroll
+  for (int f = 0; f < 4; f++)
+    net[f] = nb[f] == iel ? negF(fm[f]) : cget(F.fcdm, nb[f], fc[f]) - fm[f];
+  const double totm = (net[0] + net[2]) + (net[1] + net[3]);
+  const double cnfl = quarter(totm);
+  const double c02 = quarter(net[0] - net[2]), c13 = quarter(net[1] - net[3]);
+  const double cndm[4] = {c02, c13, c02, c13};
+#else
   double nfm[4];
   double totm = 0.0;
 #pragma unroll
@@ -234,24 +299,6 @@ __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
     if (nb[i2] == iel) w2 = 0.0;
     totm = totm - fm[i1] - fm[i2] + w1 + w2;
   }
-  const double totv = F.cutm_el[iel];
-  // ale_kn_updatebasisel
-  const double vpr = F.vol[iel], mpr = F.mass[iel];
-  const double v1 = vpr + totv;
-  const double m1 = mpr + totm;
-  F.vpr[iel] = vpr;
-  F.mpr[iel] = mpr;
-  F.vol[iel] = v1;
-  F.mass[iel] = m1;
-  F.rho[iel] = DIV(m1, v1);
-  // ale_kn_fluxelvl(cnmass, fcdm, elenergy)
-  const d4 cm = F.cnmass[iel];
-  const double ob[4] = {cm.x, cm.y, cm.z, cm.w};
-  const double ev = F.e[iel];
-  double ef[4];
-  elvl_pair(iel, 0, nb, fc, F.cnmass, ob, fm[0], fm[2], F.e, ev, ef[0], ef[2]);
-  elvl_pair(iel, 1, nb, fc, F.cnmass, ob, fm[1], fm[3], F.e, ev, ef[1], ef[3]);
-  F.eflux[iel] = make_d4(ef[0], ef[1], ef[2], ef[3]);
   // ale_kn_fluxbasisnd: corner mass-flux basis and corner mass flux
   double cndm[4], cnfl = 0.0;
 #pragma unroll
@@ -268,7 +315,21 @@ __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
     w3 = quarter(w1 + w2);
     cnfl = cnfl + w3;
   }
-  F.cnflux[iel] = make_d4(cnfl, cnfl, cnfl, cnfl);
+#endif
+  // ale_kn_updatebasisel: the new mass; the advected volume and its density
+  // are never read (k_ale_update forms both from the remapped vertices), so
+  // F.vol keeps the volume before the remap until then
+  F.mpr[iel] = mpr;
+  F.mass[iel] = mpr + totm;
+  F.cnflux[iel] = cnfl;  // the same for the four corners
+  // ale_kn_fluxelvl(cnmass, fcdm, elenergy)
+  const d4 cm = F.cnmass[iel];
+  const double ob[4] = {cm.x, cm.y, cm.z, cm.w};
+  const double ev = F.e[iel];
+  double ef[4];
+  elvl_pair(0, nb, fc, F.cnmass, ob, fm[0], fm[2], F.e, ev, ef[0], ef[2]);
+  elvl_pair(1, nb, fc, F.cnmass, ob, fm[1], fm[3], F.e, ev, ef[1], ef[3]);
+  F.eflux[iel] = make_d4(ef[0], ef[1], ef[2], ef[3]);
   // ale_kn_fluxndvl for u and v (ale_kn_advectors.f90:83-153): corner flux
   // pairs (ilndl, ilndr, ii) in loop order (ilfcl, icn) = (1,1),(1,2),(2,1),(2,2)
   const int4 nd = __ldg(F.ielnd + iel);
@@ -279,7 +340,11 @@ __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
     cu[j] = F.ndu[n[j]];
     cv[j] = F.ndv[n[j]];
   }
+#if BL_FAST_ALGEBRA
+  double du[2][2], dv[2][2];  // the pairs' fluxes; each corner is in two pairs
+#else
   double fu[4] = {0.0, 0.0, 0.0, 0.0}, fv[4] = {0.0, 0.0, 0.0, 0.0};
+#endif
 #pragma unroll
   for (int ilfcl = 0; ilfcl < 2; ilfcl++) {
     const int ilfcr = ilfcl + 2;
@@ -303,30 +368,19 @@ __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
       const bool lft = gtF(cdb, 0.0);
       if (lft || gtF(0.0, cdb)) {
         const int nbe = lft ? iell : ielr;
-        const int lnl = lft ? (ifcl + icn) % 4 : (ifcr + icn - 2) % 4;
-        const int lnr = lft ? (ifcl - icn + 1) % 4 : (((ifcr - icn - 1) % 4) + 4) % 4;
-        const int nearc = lft ? ilndl : ilndr, farc = lft ? ilndr : ilndl;
-        const int4 m = __ldg(F.ielnd + nbe);
-        const int mm[4] = {m.x, m.y, m.z, m.w};
-        const int nbn = mm[lft ? lnl : lnr];
-        const double rd0 = ob[nearc] - half(absF(cdb));
+        const int lnl = lft ? (ifcl + icn) & 3 : (ifcr + icn - 2) & 3;
+        const int lnr = lft ? (ifcl - icn + 1) & 3 : (ifcr - icn - 1) & 3;
+        const int nbn = node_at(__ldg(F.ielnd + nbe), lft ? lnl : lnr);
+        const double rd0 = (lft ? ob[ilndl] : ob[ilndr]) - half(absF(cdb));
         const double w5 = ob[ilndl] + ob[ilndr];
         const double w6 = cget(F.cnmass, nbe, lnl) + cget(F.cnmass, nbe, lnr);
-        const double den = w5 * w6 * (w5 + w6);
 #pragma unroll
         for (int q = 0; q < 2; q++) {
           const double* cvar = q == 0 ? cu : cv;
-          const double* nvar = q == 0 ? F.ndu : F.ndv;
-          const double rv = cvar[nearc];
-          const double I = cvar[farc] - rv, O = rv - nvar[nbn];
-#if BL_MIXED
-          const double grad = grad_f32(I, O, w5, w6, I);
-          (void)den;
-#else
-          const double w8 = DIV(I * w6 * w6 + O * w5 * w5, den);
-          double grad = sign_of(minF(minF(absF(w8), DIV(absF(O), w6)), DIV(absF(I), w5)), I);
-          if (prod_le0(O, I)) grad = 0.0;
-#endif
+          const double rv = lft ? cvar[ilndl] : cvar[ilndr];
+          const double I = (lft ? cvar[ilndr] : cvar[ilndl]) - rv;
+          const double O = rv - (q == 0 ? F.ndu : F.ndv)[nbn];
+          const double grad = limited_slope(I, O, w5, w6, I);
           const double rd = cdb * (rv + grad * rd0);
           if (q == 0) rdu = rd; else rdv = rd;
         }
@@ -381,14 +435,28 @@ __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
         }
       }
 #endif
+#if BL_FAST_ALGEBRA
+      du[ilfcl][icn - 1] = rdu;
+      dv[ilfcl][icn - 1] = rdv;
+#else
       fu[ilndl] = fu[ilndl] - rdu;
       fu[ilndr] = fu[ilndr] + rdu;
       fv[ilndl] = fv[ilndl] - rdv;
       fv[ilndr] = fv[ilndr] + rdv;
+#endif
     }
   }
+#if BL_FAST_ALGEBRA
+  // pairs (left, right): (0,3), (1,2) and (1,0), (2,3); the left corner
+  // loses what the right one gains
+  F.cnfu[iel] = make_d4(du[1][0] - du[0][0], -(du[0][1] + du[1][0]), du[0][1] - du[1][1],
+                        du[0][0] + du[1][1]);
+  F.cnfv[iel] = make_d4(dv[1][0] - dv[0][0], -(dv[0][1] + dv[1][0]), dv[0][1] - dv[1][1],
+                        dv[0][0] + dv[1][1]);
+#else
   F.cnfu[iel] = make_d4(fu[0], fu[1], fu[2], fu[3]);
   F.cnfv[iel] = make_d4(fv[0], fv[1], fv[2], fv[3]);
+#endif
   (void)zc;
 }
 
@@ -401,24 +469,40 @@ __global__ void __launch_bounds__(BS) k_ale_nd(DevFields F, DevCfg C) {
   const DevStep* S = nd_step<BATCH>(F, ind);
   if (halted_a(S) || !ale_on(C, S)) return;
   const double dt = S->dt;
-  // calcbasisnd + massbasisnd in element-major (ielsort2) order
-  double v0 = 0.0, m0 = 0.0;
+  // calcbasisnd, massbasisnd and the momentum sums in element-major
+  // (ielsort2) order, each in its own sum: m1 adds the corners' mass fluxes
+  // to the finished m0, so those are kept (a node of more than kKept
+  // corners reads the rest again).  The quarter volumes are summed as
+  // volumes, a quarter of the sum being the same bits.
+  constexpr int kKept = 4;
+  double v0 = 0.0, m0 = 0.0, fu = 0.0, fv = 0.0, cf[kKept];
   const int b = __ldg(F.ne_off + ind), e = __ldg(F.ne_off + ind + 1);
-  for (int k = b; k < e; k++) {
-    const int c = __ldg(F.ne_ent + k);
-    const int iel = c >> 2, j = c & 3;
-    v0 = v0 + quarter(F.vpr[iel]);
-    m0 = m0 + cget(F.cnmass, iel, j);
+#pragma unroll
+  for (int i = 0; i < kKept; i++) {
+    if (b + i < e) {
+      const int c = __ldg(F.ne_ent + b + i);
+      const int iel = c >> 2, j = c & 3;
+      v0 = v0 + F.vol[iel];
+      m0 = m0 + cget(F.cnmass, iel, j);
+      cf[i] = F.cnflux[iel];
+      fu = fu + cget(F.cnfu, iel, j);
+      fv = fv + cget(F.cnfv, iel, j);
+    }
   }
-  double m1 = m0;
-  double fu = 0.0, fv = 0.0;
-  for (int k = b; k < e; k++) {
+  for (int k = b + kKept; k < e; k++) {
     const int c = __ldg(F.ne_ent + k);
     const int iel = c >> 2, j = c & 3;
-    m1 = m1 + cget(F.cnflux, iel, j);
+    v0 = v0 + F.vol[iel];
+    m0 = m0 + cget(F.cnmass, iel, j);
     fu = fu + cget(F.cnfu, iel, j);
     fv = fv + cget(F.cnfv, iel, j);
   }
+  v0 = quarter(v0);
+  double m1 = m0;
+#pragma unroll
+  for (int i = 0; i < kKept; i++)
+    if (b + i < e) m1 = m1 + cf[i];
+  for (int k = b + kKept; k < e; k++) m1 = m1 + F.cnflux[__ldg(F.ne_ent + k) >> 2];
   const double cutm = C.dencut * v0;
   const int t = __ldg(F.indtype + ind);
   // ale_kn_activend(-1) / (-2) with indstatus = 2 (zeul)
@@ -449,6 +533,13 @@ __global__ void __launch_bounds__(BS) k_ale_update(DevFields F, DevCfg C) {
   // ale_kn_updateel: sumflux(flux) then the mass-weighted energy
   const d4 f4 = F.eflux[iel];
   const double ef[4] = {f4.x, f4.y, f4.z, f4.w};
+#if BL_FAST_ALGEBRA
+  double net[4];
+#pragma unroll
+  for (int f = 0; f < 4; f++)
+    net[f] = nb[f] == iel ? negF(ef[f]) : cget(F.eflux, nb[f], fc[f]) - ef[f];
+  const double elf = (net[0] + net[2]) + (net[1] + net[3]);
+#else
   double elf = 0.0;
 #pragma unroll
   for (int i1 = 0; i1 < 2; i1++) {
@@ -459,13 +550,15 @@ __global__ void __launch_bounds__(BS) k_ale_update(DevFields F, DevCfg C) {
     if (nb[i2] == iel) w2 = 0.0;
     elf = elf - ef[i1] - ef[i2] + w1 + w2;
   }
+#endif
   const double m1 = F.mass[iel], mpr = F.mpr[iel];
-  const double cut = F.vpr[iel] * C.dencut;
+  const double cut = F.vol[iel] * C.dencut;
   double e = F.e[iel];
   if (gtF(m1, cut)) e = DIV(e * mpr + elf, m1);
   // new corner masses (ale_kn_massbasisnd)
-  const d4 cm = F.cnmass[iel], cf = F.cnflux[iel];
-  F.cnmass[iel] = make_d4(cm.x + cf.x, cm.y + cf.y, cm.z + cf.z, cm.w + cf.w);
+  const d4 cm = F.cnmass[iel];
+  const double cf = F.cnflux[iel];
+  F.cnmass[iel] = make_d4(cm.x + cf, cm.y + cf, cm.z + cf, cm.w + cf);
   // ale_dr_hydroupdate: geometry at the remapped vertices, density, EoS
   const int4 nd = __ldg(F.ielnd + iel);
   const int n[4] = {nd.x, nd.y, nd.z, nd.w};

@@ -515,15 +515,12 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
   F.cnwt_h = dalloc<d4>(x, nel, st);
   if (c.zsp) F.spmass = dalloc<d4>(x, nel, st);
   if (c.ale_zexist) {
-    F.fcdv = dalloc<d4>(x, nel, st);
     F.fcdm = dalloc<d4>(x, nel, st);
     F.eflux = dalloc<d4>(x, nel, st);
-    F.cnflux = dalloc<d4>(x, nel, st);
+    F.cnflux = dalloc<double>(x, nel, st);
     F.cnfu = dalloc<d4>(x, nel, st);
     F.cnfv = dalloc<d4>(x, nel, st);
-    F.vpr = dalloc<double>(x, nel, st);
     F.mpr = dalloc<double>(x, nel, st);
-    F.cutm_el = dalloc<double>(x, nel, st);
   }
   {
     const int nblk = x->L.getdt_grid(nel);

@@ -96,12 +96,11 @@ struct DevFields {
   const int* ne_off;
   const int* ne_ent;
   // node fields
-  double *ndx, *ndy, *ndu, *ndv, *ndubar, *ndvbar, *ndxn, *ndyn;
+  double *ndx, *ndy, *ndu, *ndv, *ndubar, *ndvbar;
   // element fields
   double *rho, *e, *p, *cs2, *cs2v, *vol, *mass, *visc;
   double *a1, *a2, *a3, *b1, *b2, *b3;
   double *rho_h;             // half-step density (predictor -> node kernel)
-  double* e_scr;             // elenergy0 / ALE scratch
   // corner fields
   d4 *cnwt, *cnmass, *cnviscx, *cnviscy, *cnfx, *cnfy, *spmass;
   d4* cnwt_h;           // half-step corner volumes
@@ -113,9 +112,8 @@ struct DevFields {
   double *cprho, *cpe, *cpp, *cpcs2, *cpvol, *frvol, *cpm, *frm, *cpvisc;
   d4 *cpviscx, *cpviscy, *cpfx, *cpfy;
   // ALE scratch
-  d4 *fcdv, *fcdm, *eflux, *cndm, *cnflux, *cnfu, *cnfv, *cnm0, *cnmass_new;
-  double *vpr, *mpr, *cutm_el;
-  double* rscr25;            // split-advection stale-scratch emulation (unused)
+  d4 *fcdm, *eflux, *cnfu, *cnfv;
+  double *mpr, *cnflux;
   // edges (fast build; bl_setup.cuh): slots of unique edges, each
   // with its nodes, elements and the edges that continue it, and each
   // element's four slots
