@@ -195,11 +195,11 @@ template <int BS, bool BATCH>
 __global__ void __launch_bounds__(BS) k_ale_flux(DevFields F, DevCfg C) {
   const int iel = blockIdx.x * BS + threadIdx.x;
   if (iel >= F.nel) return;
+  const int4 nd = __ldg(F.ielnd + iel);
   DevStep* S = el_step<BATCH>(F, iel);
   if (halted_a(S) || !ale_on(C, S)) return;
   const double dt = S->dt;
   const double zc = C.zerocut;
-  const int4 nd = __ldg(F.ielnd + iel);
   const int n[4] = {nd.x, nd.y, nd.z, nd.w};
 #if BL_FAST_ALGEBRA
   // Fast build: the face's swept volume from the face vector (Dx, Dy) and
@@ -262,10 +262,10 @@ template <int BS, bool BATCH>
 __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
   const int iel = blockIdx.x * BS + threadIdx.x;
   if (iel >= F.nel) return;
+  const int4 ee = __ldg(F.ielel + iel);
   DevStep* S = el_step<BATCH>(F, iel);
   if (halted_a(S) || !ale_on(C, S)) return;
   const double zc = C.zerocut;
-  const int4 ee = __ldg(F.ielel + iel);
   const int nb[4] = {ee.x, ee.y, ee.z, ee.w};
   const int fcp = __ldg(F.ielfc + iel);
   const int fc[4] = {fc_of(fcp, 0), fc_of(fcp, 1), fc_of(fcp, 2), fc_of(fcp, 3)};
@@ -466,6 +466,7 @@ template <int BS, bool BATCH>
 __global__ void __launch_bounds__(BS) k_ale_nd(DevFields F, DevCfg C) {
   const int ind = blockIdx.x * BS + threadIdx.x;
   if (ind >= F.nnd) return;
+  const int b = __ldg(F.ne_off + ind), e = __ldg(F.ne_off + ind + 1);
   const DevStep* S = nd_step<BATCH>(F, ind);
   if (halted_a(S) || !ale_on(C, S)) return;
   const double dt = S->dt;
@@ -476,7 +477,6 @@ __global__ void __launch_bounds__(BS) k_ale_nd(DevFields F, DevCfg C) {
   // volumes, a quarter of the sum being the same bits.
   constexpr int kKept = 4;
   double v0 = 0.0, m0 = 0.0, fu = 0.0, fv = 0.0, cf[kKept];
-  const int b = __ldg(F.ne_off + ind), e = __ldg(F.ne_off + ind + 1);
 #pragma unroll
   for (int i = 0; i < kKept; i++) {
     if (b + i < e) {
@@ -524,9 +524,9 @@ template <int BS, bool BATCH>
 __global__ void __launch_bounds__(BS) k_ale_update(DevFields F, DevCfg C) {
   const int iel = blockIdx.x * BS + threadIdx.x;
   if (iel >= F.nel) return;
+  const int4 ee = __ldg(F.ielel + iel);
   DevStep* S = el_step<BATCH>(F, iel);
   if (halted_a(S) || !ale_on(C, S)) return;
-  const int4 ee = __ldg(F.ielel + iel);
   const int nb[4] = {ee.x, ee.y, ee.z, ee.w};
   const int fcp = __ldg(F.ielfc + iel);
   const int fc[4] = {fc_of(fcp, 0), fc_of(fcp, 1), fc_of(fcp, 2), fc_of(fcp, 3)};
@@ -551,6 +551,7 @@ __global__ void __launch_bounds__(BS) k_ale_update(DevFields F, DevCfg C) {
     elf = elf - ef[i1] - ef[i2] + w1 + w2;
   }
 #endif
+  const EosTab mat = eos_tab(C, __ldg(F.ielmat + iel));
   const double m1 = F.mass[iel], mpr = F.mpr[iel];
   const double cut = F.vol[iel] * C.dencut;
   double e = F.e[iel];
@@ -572,7 +573,7 @@ __global__ void __launch_bounds__(BS) k_ale_update(DevFields F, DevCfg C) {
   if (gtF(0.0, g.vol)) atomicMax(&S->negvol_ale, iel + 1 - el_base<BATCH>(F, iel));
   const double rho = DIV(m1, g.vol);
   double p, cs2;
-  eos_pc(C, __ldg(F.ielmat + iel), rho, e, p, cs2);
+  eos_pc(C, mat, rho, e, p, cs2);
   F.a1[iel] = g.a1;
   F.a2[iel] = g.a2;
   F.a3[iel] = g.a3;

@@ -110,14 +110,27 @@ namespace BL_NS {
 
 // ------------------------------------------------------------------ EoS
 // eos_kn_getpressure / eos_kn_getcs2 (eos_kn_forms.f90:28-106)
-__device__ __forceinline__ void eos_pc(const DevCfg& C, int mat, double rho, double e,
+// (the material's table entries first: they hang on the material number and
+// are asked for before the work whose result they meet)
+struct EosTab {
+  int mat, type;
+  double gm1, ggm1;
+};
+__device__ __forceinline__ EosTab eos_tab(const DevCfg& C, int mat) {
+  EosTab t;
+  t.mat = mat > 0 ? mat : 0;
+  t.type = __ldg(C.eos_type + t.mat);
+  t.gm1 = __ldg(C.eos_gm1 + t.mat);
+  t.ggm1 = __ldg(C.eos_ggm1 + t.mat);
+  return t;
+}
+__device__ __forceinline__ void eos_pc(const DevCfg& C, const EosTab& T, double rho, double e,
                                        double& p, double& cs2) {
-  const int imat = mat > 0 ? mat : 0;
-  const int t = __ldg(C.eos_type + imat);
-  const double* P = C.eos_param + 6 * imat;
+  const int t = T.type;
+  const double* P = C.eos_param + 6 * T.mat;
   if (t == 1) {
-    p = e * rho * __ldg(C.eos_gm1 + imat);
-    cs2 = __ldg(C.eos_ggm1 + imat) * e;
+    p = e * rho * T.gm1;
+    cs2 = T.ggm1 * e;
   } else if (t == 0) {
     p = __ldg(P);
     cs2 = C.ccut;
@@ -151,6 +164,11 @@ __device__ __forceinline__ void eos_pc(const DevCfg& C, int mat, double rho, dou
   }
   if (gt_nn(C.pcut, absF(p))) p = 0.0;
   cs2 = maxF(cs2, C.ccut);
+}
+
+__device__ __forceinline__ void eos_pc(const DevCfg& C, int mat, double rho, double e, double& p,
+                                       double& cs2) {
+  eos_pc(C, eos_tab(C, mat), rho, e, p, cs2);
 }
 
 // ------------------------------------------------------------------ geometry
@@ -543,8 +561,9 @@ __device__ __forceinline__ void getdt_div(const DevFields& F, int iel, const dou
 }
 
 // hydro_dr_getcs2: elcs2 += elvisc; mixed cells: sum frmass*(cpcs2+cpvisc)
-__device__ __forceinline__ double signal_speed(const DevFields& F, int iel, double visc) {
-  double cs2v = F.cs2[iel] + visc;
+__device__ __forceinline__ double signal_speed(const DevFields& F, int iel, double cs2,
+                                               double visc) {
+  double cs2v = cs2 + visc;
   const int imx = F.elmx ? F.elmx[iel] : -1;
   if (imx >= 0) {
     double w1 = 0.0;
@@ -559,7 +578,7 @@ __device__ __forceinline__ double signal_speed(const DevFields& F, int iel, doub
 // the element's CFL candidate from its squared length len (getdt_cfl_len)
 __device__ __forceinline__ void getdt_cfl(const DevFields& F, int iel, double len, double visc,
                                           double& cflv, int& cfli) {
-  const double cs2v = signal_speed(F, iel, visc);
+  const double cs2v = signal_speed(F, iel, F.cs2[iel], visc);
 #if BL_MIXED
   const double r11 = len < 0.0 ? DBL_MAX : from_lr(DIV(to_lr(len), to_lr(cs2v)));
 #else
@@ -584,62 +603,102 @@ __device__ __forceinline__ void getdt_tail(const DevFields& F, const DevCfg& C, 
   getdt_div(F, iel, u, v, divv, divi);
 }
 
+// A warp's smallest CFL candidate and largest divergence candidate, in every
+// lane, by integer reductions: the values as order keys, high word, then low
+// word among the lanes that hold it, then the first element number among
+// those.  The rules are cfl_min's and div_max's; a NaN never is the smallest.
+__device__ __forceinline__ void warp_cfl_min(double& v, int& i) {
+  const unsigned all = 0xffffffffu;
+  const unsigned long long k =
+      nanF(v) ? ~0ull : (unsigned long long)okey(v) ^ 0x8000000000000000ull;
+  const unsigned hi = __reduce_min_sync(all, (unsigned)(k >> 32));
+  const bool h = (unsigned)(k >> 32) == hi;
+  const unsigned lo = __reduce_min_sync(all, h ? (unsigned)k : all);
+  const bool l = h && (unsigned)k == lo;
+  const int at = __ffs(__ballot_sync(all, l)) - 1;
+  i = __reduce_min_sync(all, l ? i : 0x7fffffff);
+  v = from_bits64(((long long)__shfl_sync(all, (int)(bits64(v) >> 32), at) << 32) |
+                  (unsigned)__shfl_sync(all, (int)bits64(v), at));
+}
+__device__ __forceinline__ void warp_div_max(double& v, int& i) {
+  const unsigned all = 0xffffffffu;
+  const unsigned long long k = (unsigned long long)bits64(v);
+  const unsigned hi = __reduce_max_sync(all, (unsigned)(k >> 32));
+  const bool h = (unsigned)(k >> 32) == hi;
+  const unsigned lo = __reduce_max_sync(all, h ? (unsigned)k : 0u);
+  const bool l = h && (unsigned)k == lo;
+  const int m = __reduce_min_sync(all, l && i >= 0 ? i : 0x7fffffff);
+  i = m == 0x7fffffff ? -1 : m;
+  v = from_bits64((long long)(((unsigned long long)hi << 32) | lo));
+}
+// the same over a block, in every thread
+template <int BS>
+__device__ __forceinline__ void block_candidates(double& cflv, int& cfli, double& divv, int& divi,
+                                                 double* s_v, int* s_i) {
+  warp_cfl_min(cflv, cfli);
+  warp_div_max(divv, divi);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) {
+    s_v[2 * wid] = cflv;
+    s_v[2 * wid + 1] = divv;
+    s_i[2 * wid] = cfli;
+    s_i[2 * wid + 1] = divi;
+  }
+  __syncthreads();
+  const int w = lane < BS / 32 ? lane : 0;
+  cflv = s_v[2 * w];
+  divv = s_v[2 * w + 1];
+  cfli = s_i[2 * w];
+  divi = s_i[2 * w + 1];
+  warp_cfl_min(cflv, cfli);
+  warp_div_max(divv, divi);
+}
+
 // The block reduction of the candidates, the last block's reduction of the
 // block partials and time_dr_end (time_dr_advance.f90:74-132)
 // over the k_getdt blocks [blk0, blk0 + nblk) of one mesh (all of them for
 // a single mesh; a batch's mesh in a batch, whose time-step parameters then
-// come from I, and whose element numbers start at el0)
+// come from I, and whose element numbers start at el0).
+// This is a serial tail that every step waits for -- on a small mesh half
+// of the kernel (12,300 of 23,400 cycles at 1,000 elements) -- so it is cut
+// to dependent latencies: reductions in the integer unit's warp instructions
+// instead of five rounds of shuffles, one acquire-release ticket instead of
+// a fence and a ticket, the step header read before the ticket, the square
+// root and the divide in two warps at once, and the candidates' reciprocals
+// in five lanes while the smallest is found: 7,700 cycles.
 template <int BS, bool BATCH>
 __device__ __forceinline__ void getdt_finish(const DevFields& F, const DevCfg& C, DevStep* S,
                                              double cflv, int cfli, double divv, int divi,
                                              int blk0, int nblk, int el0, const DevInst* I) {
-  // ---- block reduction
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    double ov = __shfl_xor_sync(0xffffffffu, cflv, o);
-    int oi = __shfl_xor_sync(0xffffffffu, cfli, o);
-    cfl_min(cflv, cfli, ov, oi);
-    ov = __shfl_xor_sync(0xffffffffu, divv, o);
-    oi = __shfl_xor_sync(0xffffffffu, divi, o);
-    div_max(divv, divi, ov, oi);
-  }
-  __shared__ double s_cv[BS / 32], s_dv[BS / 32];
-  __shared__ int s_ci[BS / 32], s_di[BS / 32];
+  static_assert(BS >= 64 && BS / 32 <= 32, "two warps at least");
+  __shared__ double s_v[2][2 * (BS / 32)], s_rdt[2];
+  __shared__ int s_i[2][2 * (BS / 32)];
   __shared__ bool s_last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) {
-    s_cv[wid] = cflv;
-    s_ci[wid] = cfli;
-    s_dv[wid] = divv;
-    s_di[wid] = divi;
-  }
-  __syncthreads();
+  // the header as it is until the last block writes it
+  const double dt0 = S->dt, time0 = S->time;
+  const int nstep0 = S->nstep, run_mode = S->run_mode, nrec0 = S->nrecord;
+  block_candidates<BS>(cflv, cfli, divv, divi, s_v[0], s_i[0]);
   if (threadIdx.x == 0) {
-    for (int w = 1; w < BS / 32; w++) {
-      cfl_min(cflv, cfli, s_cv[w], s_ci[w]);
-      div_max(divv, divi, s_dv[w], s_di[w]);
-    }
-    F.red_v[2 * blockIdx.x] = cflv;
-    F.red_i[2 * blockIdx.x] = cfli;
-    F.red_v[2 * blockIdx.x + 1] = divv;
-    F.red_i[2 * blockIdx.x + 1] = divi;
-    __threadfence();
-    unsigned int t = atomicAdd(&S->ticket, 1u);
+    reinterpret_cast<double2*>(F.red_v)[blockIdx.x] = make_double2(cflv, divv);
+    reinterpret_cast<int2*>(F.red_i)[blockIdx.x] = make_int2(cfli, divi);
+    unsigned int t;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;"
+                 : "=r"(t) : "l"(&S->ticket) : "memory");
     s_last = (t == (unsigned int)(nblk - 1));
   }
   __syncthreads();
   if (!s_last) return;
   // ---- last block: reduce the partials, then time_dr_end
-  __threadfence();
   cflv = HUGE_VAL;
   cfli = 0x7fffffff;
   divv = DBL_MIN;
   divi = -1;
-  // Each thread takes the partials b = tid, tid + BS, ... in that order as
-  // before, eight at a time: their loads (L2, past the L1 that may not see
-  // other blocks' writes) are all in flight before the first comparison.
-  // (Sixteen at a time, one round fewer on a 512x512 mesh, spilled in the
-  // rest of the kernel and made it slower.)
+  // Each thread takes the partials b = tid, tid + BS, ..., eight at a time:
+  // their loads (L2, past the L1 that may not see other blocks' writes) are
+  // all in flight before the first comparison.  (Sixteen at a time, one
+  // round fewer on a 512x512 mesh, spilled in the rest of the kernel and
+  // made it slower.)
   {
     constexpr int U = 8;
     const double2* rv = reinterpret_cast<const double2*>(F.red_v) + blk0;
@@ -665,83 +724,77 @@ __device__ __forceinline__ void getdt_finish(const DevFields& F, const DevCfg& C
       }
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    double ov = __shfl_xor_sync(0xffffffffu, cflv, o);
-    int oi = __shfl_xor_sync(0xffffffffu, cfli, o);
-    cfl_min(cflv, cfli, ov, oi);
-    ov = __shfl_xor_sync(0xffffffffu, divv, o);
-    oi = __shfl_xor_sync(0xffffffffu, divi, o);
-    div_max(divv, divi, ov, oi);
-  }
-  __syncthreads();
+  block_candidates<BS>(cflv, cfli, divv, divi, s_v[1], s_i[1]);
+  // one thread's operations: the hardware's correctly rounded square root
+  // and divide (the same results as the integer-pipe routines, at less
+  // latency)
   if (lane == 0) {
-    s_cv[wid] = cflv;
-    s_ci[wid] = cfli;
-    s_dv[wid] = divv;
-    s_di[wid] = divi;
+    if (wid == 0) s_rdt[0] = C.cfl_sf * sqrt(cflv);
+    else if (wid == 1) s_rdt[1] = C.div_sf / divv;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  for (int w = 1; w < BS / 32; w++) {
-    cfl_min(cflv, cfli, s_cv[w], s_ci[w]);
-    div_max(divv, divi, s_dv[w], s_di[w]);
-  }
-  S->ticket = 0;
+  if (wid != 0) return;
+  if (lane == 0) S->ticket = 0;
   // time_dr_calc candidates then hydro's CFL and DIV (time_dr_advance.f90)
   if (cflv < 0.0) {  // hydro_kn_getdtcfl FAILURE
+    if (lane != 0) return;
     S->ierr = -1;
     S->iout = 2;
     S->err_code = 1;
-    if (S->run_mode) S->halted = 1;
+    if (run_mode) S->halted = 1;
     return;
   }
-  // one thread's three operations: the hardware's correctly rounded
-  // square root and divide (the same results as the integer-pipe routines,
-  // at a fraction of their latency on the serial tail)
-  const double rdt_cfl = C.cfl_sf * sqrt(cflv);
-  const double rdt_div = C.div_sf / divv;
-  // 1-based element numbers local to the mesh (0: none)
-  const int cfln = cfli >= 0 && cfli != 0x7fffffff ? cfli - el0 + 1 : 0;
-  const int divn = divi >= 0 ? divi - el0 + 1 : 0;
+  const double rdt_cfl = s_rdt[0], rdt_div = s_rdt[1];
   const double dt_max = BATCH ? I->dt_max : C.dt_max, dt_g = BATCH ? I->dt_g : C.dt_g;
   const double dt_initial = BATCH ? I->dt_initial : C.dt_initial;
   const double dt_min = BATCH ? I->dt_min : C.dt_min, time_end = BATCH ? I->time_end : C.time_end;
+  // lane k holds candidate k of the reference's order and its reciprocal
+  const double g = dt_g * dt0;
+  const double mine = lane == 1 ? g : lane == 2 ? dt_initial : lane == 3 ? rdt_cfl
+                    : lane == 4 ? rdt_div : dt_max;
+  const double inv = 1.0 / mine;
+  double mind = dt_max;
+  int mins = 0;
+  if (gtF(mind, g)) { mind = g; mins = 1; }
+  if (nstep0 == 0 && gtF(mind, dt_initial)) { mind = dt_initial; mins = 2; }
+  if (gtF(mind, rdt_cfl)) { mind = rdt_cfl; mins = 3; }
+  if (gtF(mind, rdt_div)) { mind = rdt_div; mins = 4; }
+  const double rdt = __shfl_sync(0xffffffffu, inv, mins);
+  if (lane != 0) return;
+  // 1-based element numbers local to the mesh (0: none)
+  const int cfln = cfli >= 0 && cfli != 0x7fffffff ? cfli - el0 + 1 : 0;
+  const int divn = divi >= 0 ? divi - el0 + 1 : 0;
+  const int mini = mins == 3 ? cfln : (mins == 4 ? divn : -1);
+  const double time = time0 + mind;
   S->cfl_rdt = rdt_cfl;
   S->cfl_idt = cfln;
   S->div_rdt = rdt_div;
   S->div_idt = divn;
-  double mind = dt_max;
-  int mini = -1, mins = 0;
-  double g = dt_g * S->dt;
-  if (g < mind) { mind = g; mini = -1; mins = 1; }
-  if (S->nstep == 0 && dt_initial < mind) { mind = dt_initial; mini = -1; mins = 2; }
-  if (rdt_cfl < mind) { mind = rdt_cfl; mini = cfln; mins = 3; }
-  if (rdt_div < mind) { mind = rdt_div; mini = divn; mins = 4; }
-  S->nstep = S->nstep + 1;
+  S->nstep = nstep0 + 1;
   S->dt = mind;
-  S->rdt = 1.0 / mind;
+  S->rdt = rdt;
   S->sdt = mins;
   S->idtel = mini;
-  S->time = S->time + mind;
-  if (mind < dt_min) {
+  S->time = time;
+  const bool low = gtF(dt_min, mind);
+  if (low) {
     S->ierr = -1;
     S->iout = 1;
     S->err_code = 2;
-    if (S->run_mode) S->halted = 1;
+    if (run_mode) S->halted = 1;
   }
-  if (S->run_mode) {
-    if (S->time >= time_end) S->stop_next = 1;
-    int r = S->nrecord;
-    if (F.hist && r < C.max_records) {
-      F.hist[r].time = S->time;
-      F.hist[r].dt = S->dt;
-      F.hist[r].nstep = S->nstep;
-      F.hist[r].idtel = S->idtel;
-      F.hist[r].sdt_code = S->sdt;
-      F.hist[r].ierr = S->ierr;
+  if (run_mode) {
+    if (geF(time, time_end)) S->stop_next = 1;
+    if (F.hist && nrec0 < C.max_records) {
+      StepRec& r = F.hist[nrec0];
+      r.time = time;
+      r.dt = mind;
+      r.nstep = nstep0 + 1;
+      r.idtel = mini;
+      r.sdt_code = mins;
+      r.ierr = low ? -1 : S->ierr;
     }
-    S->nrecord = r + 1;
+    S->nrecord = nrec0 + 1;
   }
 }
 
@@ -1124,7 +1177,6 @@ __global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C
   const int t = threadIdx.x;
   const int slot = (int)blockIdx.x * (BS - 2) + t - 1;
   bool in = slot >= 0 && slot < F.nslot;
-  if (!BATCH && (halted(F.step) || F.step->stop_next)) return;
   int4 n = make_int4(0, 0, 0, 0), q = make_int4(-1, -1, -1, -1);
   if (in) {
     n = __ldg(F.es_n + slot);
@@ -1134,6 +1186,7 @@ __global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C
       in = !(halted(S) || S->stop_next);
     }
   }
+  if (!BATCH && (halted(F.step) || F.step->stop_next)) return;
   __shared__ double s_d[4][BS];
   EndD d = {0.0, 0.0, 0.0, 0.0};
   if (in) d = node_diff(F, n.x, n.y);
@@ -1224,10 +1277,9 @@ __global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C
 __device__ __forceinline__ double cfl_candidate(const DevFields& F, const DevCfg& C, int iel,
                                                 const double* W, const double* sq, double a1,
                                                 double a2, double a3, double b1, double b2,
-                                                double b3, double cs2v) {
-  const int ireg = __ldg(F.ielreg + iel);
-  if (__ldg(C.zdtnotreg + ireg)) return DBL_MAX;
-  if (__ldg(C.zmidlength + ireg)) {  // min over sides of |midpoint difference|^2
+                                                double b3, double cs2v, int notdt, int mid) {
+  if (notdt) return DBL_MAX;
+  if (mid) {  // min over sides of |midpoint difference|^2
     const double r0 = a3 * a3 + b3 * b3, r1 = a1 * a1 + b1 * b1;
     return DIV(times4(minF_nn(r0, r1)), cs2v);
   }
@@ -1287,24 +1339,28 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
     el0 = I->el_begin;
     el1 = I->el_end;
   }
+  const int iel = el0 + ((int)blockIdx.x - blk0) * BS + (int)threadIdx.x;
+  // (the tables' loads leave before the header's answer is needed)
+  uint4 er4 = make_uint4(0u, 0u, 0u, 0u);
+  if (iel < el1) er4 = __ldg(F.eref + iel);
   if (halted(S)) return;
   if (S->stop_next) {            // bl_run: the previous step reached time_end
     if ((int)blockIdx.x == blk0 && threadIdx.x == 0) S->halted = 1;
     return;
   }
-  const int iel = el0 + ((int)blockIdx.x - blk0) * BS + (int)threadIdx.x;
   double cflv = HUGE_VAL;        // sentinel above HUGE(1.0)
   int cfli = 0x7fffffff;
   double divv = DBL_MIN;         // TINY(1.0)
   int divi = -1;
   if (iel < el1) {
-    const uint4 er4 = __ldg(F.eref + iel);
     const unsigned er[4] = {er4.x, er4.y, er4.z, er4.w};
     double visc = 0.0;
     double du[4], dv[4], sq[4], W[4], edx[4], edy[4];
     const double a1 = F.a1[iel], a2 = F.a2[iel], a3 = F.a3[iel];
     const double b1 = F.b1[iel], b2 = F.b2[iel], b3 = F.b3[iel];
-    const double vol = F.vol[iel];
+    const double vol = F.vol[iel], rho = F.rho[iel], cs2 = F.cs2[iel];
+    const int ireg = __ldg(F.ielreg + iel);
+    const int notdt = __ldg(C.zdtnotreg + ireg), mid = __ldg(C.zmidlength + ireg);
     {
       const double cross = quarter(vol);
       const double t1 = a1 * b2 - a2 * b1, t3 = a3 * b2 - a2 * b3;
@@ -1341,15 +1397,15 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
       edy[f] = cut ? 0.0 : dv[f] * d;
     }
     if (!C.ztq) {
-      visc = DIV(twice(vmax), maxF(F.rho[iel], zc));
+      visc = DIV(twice(vmax), maxF(rho, zc));
       F.cnviscx[iel] = make_d4(edx[0] - edx[3], edx[1] - edx[0], edx[2] - edx[1], edx[3] - edx[2]);
       F.cnviscy[iel] = make_d4(edy[0] - edy[3], edy[1] - edy[0], edy[2] - edy[1], edy[3] - edy[2]);
       F.visc[iel] = visc;
     } else {
       visc = F.visc[iel];
     }
-    const double cs2v = signal_speed(F, iel, visc);
-    cflv = cfl_candidate(F, C, iel, W, sq, a1, a2, a3, b1, b2, b3, cs2v);
+    const double cs2v = signal_speed(F, iel, cs2, visc);
+    cflv = cfl_candidate(F, C, iel, W, sq, a1, a2, a3, b1, b2, b3, cs2v, notdt, mid);
     cfli = iel;
     const double w = b1 * (du[3] - du[1]) + b3 * (du[0] - du[2]) - a1 * (dv[3] - dv[1]) -
                      a3 * (dv[0] - dv[2]);
@@ -1616,12 +1672,12 @@ template <int BS, bool BATCH>
 __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, DevCfg C) {
   const int iel = blockIdx.x * BS + threadIdx.x;
   if (iel >= F.nel) return;
+  const int4 nd = __ldg(F.ielnd + iel);
   DevStep* S = el_step<BATCH>(F, iel);
   if (halted(S)) return;
   const double dt = S->dt;
   const double hdt = half(dt);   // time_dr_setpredictor dts / getvertex step
   const double zc = C.zerocut;
-  const int4 nd = __ldg(F.ielnd + iel);
   const int n[4] = {nd.x, nd.y, nd.z, nd.w};
   double u[4], v[4];
 #pragma unroll
@@ -1631,7 +1687,7 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
   }
   const d4 qx = F.cnviscx[iel], qy = F.cnviscy[iel];
   const int ireg = __ldg(F.ielreg + iel);
-  const int mat = __ldg(F.ielmat + iel);
+  const EosTab mat = eos_tab(C, __ldg(F.ielmat + iel));
   const double m = F.mass[iel];
   const double e0 = F.e[iel];
   const int imx = F.elmx ? F.elmx[iel] : -1;
@@ -1883,13 +1939,17 @@ template <int BS, bool BATCH>
 __global__ void BL_ACCEL_BOUNDS(BS) k_lag_accel(DevFields F, DevCfg C) {
   const int ind = blockIdx.x * BS + threadIdx.x;
   if (ind >= F.nnd) return;
+  const int b = __ldg(F.nc_off + ind), e = __ldg(F.nc_off + ind + 1);
   const DevStep* S = nd_step<BATCH>(F, ind);
   if (halted(S)) return;
   const double dt = S->dt;
   const double zc = C.zerocut;
+  // asked for before the gather, used after it
+  const int t = __ldg(F.indtype + ind);
+  const double u0 = F.ndu[ind], v0 = F.ndv[ind];
+  double x = F.ndx[ind], y = F.ndy[ind];
   // hydro_kn_scatteracceleration: corner-major order over ielsort
   double ndm = 0.0, nda = 0.0, fx = 0.0, fy = 0.0;
-  const int b = __ldg(F.nc_off + ind), e = __ldg(F.nc_off + ind + 1);
   for (int k = b; k < e; k++) {
     const int c = __ldg(F.nc_ent + k);
     const int iel = c >> 2, jj = c & 3;
@@ -1918,7 +1978,6 @@ __global__ void BL_ACCEL_BOUNDS(BS) k_lag_accel(DevFields F, DevCfg C) {
     ay = 0.0;
   }
   // utils_kn_bc on the accelerations
-  const int t = __ldg(F.indtype + ind);
   if (t == -1) ax = 0.0;
   else if (t == -2) ay = 0.0;
   else if (t == -3) { ax = 0.0; ay = 0.0; }
@@ -1929,10 +1988,8 @@ __global__ void BL_ACCEL_BOUNDS(BS) k_lag_accel(DevFields F, DevCfg C) {
   }
   // hydro_kn_applyacceleration, then both half vertex moves
   const double hdt = 0.5 * dt;
-  const double u0 = F.ndu[ind], v0 = F.ndv[ind];
   const double u1 = u0 + dt * ax, v1 = v0 + dt * ay;
   const double ub = u0 + hdt * ax, vb = v0 + hdt * ay;
-  double x = F.ndx[ind], y = F.ndy[ind];
   x = x + hdt * u0;
   y = y + hdt * v0;
   x = x + hdt * u1;
@@ -1951,11 +2008,11 @@ template <int BS, bool BATCH>
 __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
   const int iel = blockIdx.x * BS + threadIdx.x;
   if (iel >= F.nel) return;
+  const int4 nd = __ldg(F.ielnd + iel);
   DevStep* S = el_step<BATCH>(F, iel);
   if (halted(S)) return;
   const double dt = S->dt;
   const double zc = C.zerocut;
-  const int4 nd = __ldg(F.ielnd + iel);
   const int n[4] = {nd.x, nd.y, nd.z, nd.w};
   double x[4], y[4], ub[4], vb[4];
 #pragma unroll
@@ -1965,16 +2022,18 @@ __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
     ub[j] = F.ndubar[n[j]];
     vb[j] = F.ndvbar[n[j]];
   }
+  // asked for before the geometry, used after it
+  const EosTab mat = eos_tab(C, __ldg(F.ielmat + iel));
+  const double m = F.mass[iel], e0 = F.e[iel];
   Iso g = getiso(x, y);
   if (gtF(0.0, g.vol)) atomicMax(&S->negvol_corr, iel + 1 - el_base<BATCH>(F, iel));
-  const double m = F.mass[iel];
   const double rho = DIV(m, g.vol);
   const d4 f4x = F.cnfx[iel], f4y = F.cnfy[iel];
   const double fx[4] = {f4x.x, f4x.y, f4x.z, f4x.w};
   const double fy[4] = {f4y.x, f4y.y, f4y.z, f4y.w};
-  const double e = energy_update(F.e[iel], m, zc, dt, fx, fy, ub, vb);
+  const double e = energy_update(e0, m, zc, dt, fx, fy, ub, vb);
   double p, cs2;
-  eos_pc(C, __ldg(F.ielmat + iel), rho, e, p, cs2);
+  eos_pc(C, mat, rho, e, p, cs2);
   F.a1[iel] = g.a1;
   F.a2[iel] = g.a2;
   F.a3[iel] = g.a3;
