@@ -30,13 +30,6 @@ __device__ __forceinline__ bool halted_a(const DevStep* S) {
   return *((volatile const int*)&S->halted) != 0;
 }
 
-// ale_active (ale_dr_utils.f90:35-51)
-__device__ __forceinline__ bool ale_on(const DevCfg& C, const DevStep* S) {
-  if (!C.ale_zexist) return false;
-  const double t = S->time;
-  return geF(t, C.ale_mintime) && geF(C.ale_maxtime, t);  // the IEEE >= on the integer pipe
-}
-
 __device__ __forceinline__ int node_at(const int4& n, int j) {
   return j == 0 ? n.x : (j == 1 ? n.y : (j == 2 ? n.z : n.w));
 }
@@ -191,30 +184,54 @@ __device__ __forceinline__ void elvl_pair(int i1, const int* nb, const int* fc,
 
 // ================================================================ k_ale_flux
 
-template <int BS, bool BATCH>
+// LOOP: k_lag_state of the same step left the swept volumes of every
+// element's faces 0 and 3; a face 1 or 2 takes the one of the face across it
+// when that is a face 0 or 3 (exactly the negative), so 12 FP64 operations a
+// face are done once: Noh 1024x1024 1047 -> 997 us a step (with k_lag_state's
+// unread results left out), the demoted form 981 -> 931, a 97x97 blast 64 -> 60.
+template <int BS, bool BATCH, bool LOOP>
 __global__ void __launch_bounds__(BS) k_ale_flux(DevFields F, DevCfg C) {
   const int iel = blockIdx.x * BS + threadIdx.x;
   if (iel >= F.nel) return;
   const int4 nd = __ldg(F.ielnd + iel);
+  const int4 ee = __ldg(F.ielel + iel);
+  const int fcp = __ldg(F.ielfc + iel);
   DevStep* S = el_step<BATCH>(F, iel);
   if (halted_a(S) || !ale_on(C, S)) return;
   const double dt = S->dt;
   const double zc = C.zerocut;
   const int n[4] = {nd.x, nd.y, nd.z, nd.w};
+  const int nb[4] = {ee.x, ee.y, ee.z, ee.w};
+  const int fc[4] = {fc_of(fcp, 0), fc_of(fcp, 1), fc_of(fcp, 2), fc_of(fcp, 3)};
+  double fv[4];
 #if BL_FAST_ALGEBRA
-  // Fast build: the face's swept volume from the face vector (Dx, Dy) and
-  // the differences and sums of the mesh velocity -ubar at its ends: the
-  // reference's quarter(a1*b3 - a3*b1) of the quad (x0(j), x0(j+1),
-  // x1(j+1), x1(j)) with x1 = x0 - dt*ubar expands (exactly in real
-  // arithmetic) to dt/4 * (2 (Dy Su - Dx Sv) + dt (Du Sv - Dv Su)), which
-  // also avoids the cancellation of subtracting positions at two times.
-  double x0[4], y0[4], ub[4], vb[4];
+  if (LOOP) {
+    fv[0] = F.fdv0[iel];
+    fv[3] = F.fdv3[iel];
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    x0[j] = F.ndx[n[j]];
-    y0[j] = F.ndy[n[j]];
-    ub[j] = F.ndubar[n[j]];
-    vb[j] = F.ndvbar[n[j]];
+    for (int j = 1; j <= 2; j++) {
+      if (nb[j] != iel && (fc[j] == 0 || fc[j] == 3)) {
+        fv[j] = negF((fc[j] == 0 ? F.fdv0 : F.fdv3)[nb[j]]);
+      } else {
+        const int a = n[j], b = n[j + 1];
+        fv[j] = swept(F.ndx[a], F.ndy[a], F.ndubar[a], F.ndvbar[a], F.ndx[b], F.ndy[b],
+                      F.ndubar[b], F.ndvbar[b], dt);
+      }
+    }
+  } else {
+    double x0[4], y0[4], ub[4], vb[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      x0[j] = F.ndx[n[j]];
+      y0[j] = F.ndy[n[j]];
+      ub[j] = F.ndubar[n[j]];
+      vb[j] = F.ndvbar[n[j]];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int k = (j + 1) & 3;
+      fv[j] = swept(x0[j], y0[j], ub[j], vb[j], x0[k], y0[k], ub[k], vb[k], dt);
+    }
   }
 #else
   double x0[4], y0[4], x1[4], y1[4];
@@ -226,26 +243,14 @@ __global__ void __launch_bounds__(BS) k_ale_flux(DevFields F, DevCfg C) {
     x1[j] = x0[j] + dt * (-F.ndubar[n[j]]);
     y1[j] = y0[j] + dt * (-F.ndvbar[n[j]]);
   }
-#endif
-  double fv[4];
 #pragma unroll
-  for (int jj = 0; jj < 4; jj++) {
-    const int jp = (jj + 1) & 3;
-#if BL_FAST_ALGEBRA
-    const double Dx = x0[jp] - x0[jj], Dy = y0[jp] - y0[jj];
-    const double Du = ub[jp] - ub[jj], Dv = vb[jp] - vb[jj];
-    const double Su = ub[jp] + ub[jj], Sv = vb[jp] + vb[jj];
-    const double A = Dy * Su - Dx * Sv, B = Du * Sv - Dv * Su;
-    double d = quarter(dt * fma(dt, B, twice(A)));
-#else
-    double d = face_dv(x0[jj], x0[jp], y0[jj], y0[jp], x1[jp], x1[jj], y1[jp], y1[jj]);
-#endif
-    fv[jj] = gtF(zc, d) ? 0.0 : d;
+  for (int j = 0; j < 4; j++) {
+    const int k = (j + 1) & 3;
+    fv[j] = face_dv(x0[j], x0[k], y0[j], y0[k], x1[k], x1[j], y1[k], y1[j]);
   }
-  const int4 ee = __ldg(F.ielel + iel);
-  const int nb[4] = {ee.x, ee.y, ee.z, ee.w};
-  const int fcp = __ldg(F.ielfc + iel);
-  const int fc[4] = {fc_of(fcp, 0), fc_of(fcp, 1), fc_of(fcp, 2), fc_of(fcp, 3)};
+#endif
+#pragma unroll
+  for (int j = 0; j < 4; j++) fv[j] = gtF(zc, fv[j]) ? 0.0 : fv[j];
   // ale_kn_fluxelvl(cnwt, fcdv, eldensity)
   const d4 cw = F.cnwt[iel];
   const double ob[4] = {cw.x, cw.y, cw.z, cw.w};
@@ -611,7 +616,8 @@ static constexpr int BS_AN = 256;
 template <bool BATCH>
 void launch_ale_t(const DevFields& F, const DevCfg& C, cudaStream_t s) {
   const int ge = (F.nel + BS_A - 1) / BS_A;
-  k_ale_flux<BS_A, BATCH><<<ge, BS_A, 0, s>>>(F, C);
+  if (F.loop_ale) k_ale_flux<BS_A, BATCH, true><<<ge, BS_A, 0, s>>>(F, C);
+  else k_ale_flux<BS_A, BATCH, false><<<ge, BS_A, 0, s>>>(F, C);
   k_ale_el<BS_A, BATCH><<<ge, BS_A, 0, s>>>(F, C);
   if constexpr (!BATCH) {
     k_ale_nd<BS_AN, false><<<(F.nnd + BS_AN - 1) / BS_AN, BS_AN, 0, s>>>(F, C);

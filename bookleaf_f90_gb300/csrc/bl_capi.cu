@@ -523,6 +523,8 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
     F.cnfu = dalloc<d4>(x, nel, st);
     F.cnfv = dalloc<d4>(x, nel, st);
     F.mpr = dalloc<double>(x, nel, st);
+    F.fdv0 = dalloc<double>(x, nel, st);
+    F.fdv3 = dalloc<double>(x, nel, st);
   }
   {
     const int nblk = x->L.getdt_grid(nel);
@@ -838,6 +840,7 @@ int bl_run(bl_ctx* x, bl_timestep* ts, int max_steps, bl_step_record* history, i
   if (!history) F.hist = nullptr;
   C.max_records = history ? x->hist_cap : 0;
   const bool with_ale = x->c.ale_zexist != 0;
+  F.loop_ale = with_ale;
   const int G = 16;  // steps per graph launch
   if (!x->gexec || x->gsteps != G || x->g_ale != with_ale || x->g_hist != F.hist ||
       x->g_maxrec != C.max_records) {
@@ -1688,6 +1691,7 @@ int bl_run_batch(bl_ctx* x, bl_timestep* ts, int max_steps, int* status, int* ns
   cudaError_t r;
   bl::DevFields F = x->F;
   F.hist = nullptr;
+  F.loop_ale = with_ale;
   bl::DevCfg C = x->C;
   C.max_records = 0;
   auto queue_step = [&]() {

@@ -114,6 +114,7 @@ struct DevFields {
   // ALE scratch
   d4 *fcdm, *eflux, *cnfu, *cnfv;
   double *mpr, *cnflux;
+  double *fdv0, *fdv3;       // swept volumes of faces 0 and 3 (device loops)
   // edges (fast build; bl_setup.cuh): slots of unique edges, each
   // with its nodes, elements and the edges that continue it, and each
   // element's four slots
@@ -137,9 +138,10 @@ struct DevFields {
   const int* blkinst;        // [nblk_batch] mesh of a k_getdt block
   int ninst, nblk_batch;
   int nd_block;              // block size of the batch's node kernels (autotuned)
+  int loop_ale;              // the launches are a device loop's that remaps
   // learned mixed-cell closure (bl_set_closure): 0 off, 1 volume and energy
   // exchange, 2 volume only
-  int closure;
+  int closure, pad0;
   float* mlp_img;            // the network's parameters as their shared-memory
                              // image (bl_mma.cuh), copied at bl_set_closure
   const float* mlp_norm;     // [22]: feature means, inverse spreads, output

@@ -2004,7 +2004,37 @@ __global__ void BL_ACCEL_BOUNDS(BS) k_lag_accel(DevFields F, DevCfg C) {
 
 // ================================================================ k_lag_state
 
-template <int BS, bool BATCH>
+// ale_active (ale_dr_utils.f90:35-51)
+__device__ __forceinline__ bool ale_on(const DevCfg& C, const DevStep* S) {
+  if (!C.ale_zexist) return false;
+  const double t = S->time;
+  return geF(t, C.ale_mintime) && geF(C.ale_maxtime, t);  // the IEEE >= on the integer pipe
+}
+
+#if BL_FAST_ALGEBRA
+// The volume an element's face sweeps in the remap, from the face vector
+// (Dx, Dy) and the differences and sums of the mesh velocity -ubar at its
+// ends (a, b): the reference's quarter(a1*b3 - a3*b1) of the quad (x0(a),
+// x0(b), x1(b), x1(a)) with x1 = x0 - dt*ubar expands (exactly in real
+// arithmetic) to dt/4 * (2 (Dy Su - Dx Sv) + dt (Du Sv - Dv Su)), which also
+// avoids the cancellation of subtracting positions at two times.  Run the
+// other way (b, a) it is exactly the negative.
+__device__ __forceinline__ double swept(double xa, double ya, double ua, double va, double xb,
+                                        double yb, double ub, double vb, double dt) {
+  const double Dx = xb - xa, Dy = yb - ya, Du = ub - ua, Dv = vb - va;
+  const double Su = ub + ua, Sv = vb + va;
+  const double A = fma(Dy, Su, -(Dx * Sv)), B = fma(Du, Sv, -(Dv * Su));
+  return quarter(dt * fma(dt, B, twice(A)));
+}
+#endif
+
+// LOOP: in a device loop whose remap follows with the same dt.  What the
+// remap then overwrites unread -- the coefficients a1..b3, pressure and sound
+// speed -- is left out, and the fast and mixed builds' kernel, which has the
+// positions and velocities at hand, leaves the swept volumes of faces 0 and 3
+// for k_ale_flux (a step called alone may be followed by anything: it does
+// all of its own work, and so does the remap).
+template <int BS, bool BATCH, bool LOOP = false>
 __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
   const int iel = blockIdx.x * BS + threadIdx.x;
   if (iel >= F.nel) return;
@@ -2032,14 +2062,23 @@ __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
   const double fx[4] = {f4x.x, f4x.y, f4x.z, f4x.w};
   const double fy[4] = {f4y.x, f4y.y, f4y.z, f4y.w};
   const double e = energy_update(e0, m, zc, dt, fx, fy, ub, vb);
-  double p, cs2;
-  eos_pc(C, mat, rho, e, p, cs2);
-  F.a1[iel] = g.a1;
-  F.a2[iel] = g.a2;
-  F.a3[iel] = g.a3;
-  F.b1[iel] = g.b1;
-  F.b2[iel] = g.b2;
-  F.b3[iel] = g.b3;
+  if (!LOOP || !ale_on(C, S)) {
+    double p, cs2;
+    eos_pc(C, mat, rho, e, p, cs2);
+    F.a1[iel] = g.a1;
+    F.a2[iel] = g.a2;
+    F.a3[iel] = g.a3;
+    F.b1[iel] = g.b1;
+    F.b2[iel] = g.b2;
+    F.b3[iel] = g.b3;
+    F.p[iel] = p;
+    F.cs2[iel] = cs2;
+  } else {
+#if BL_FAST_ALGEBRA
+    F.fdv0[iel] = swept(x[0], y[0], ub[0], vb[0], x[1], y[1], ub[1], vb[1], dt);
+    F.fdv3[iel] = swept(x[3], y[3], ub[3], vb[3], x[0], y[0], ub[0], vb[0], dt);
+#endif
+  }
   F.cnwt[iel] = make_d4(g.w0, g.w1, g.w2, g.w3);
   const int imx = F.elmx ? F.elmx[iel] : -1;
   // the learned closure (k_mix_closure, launched next) splits a two-material
@@ -2050,8 +2089,6 @@ __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
   F.vol[iel] = g.vol;
   F.rho[iel] = rho;
   F.e[iel] = e;
-  F.p[iel] = p;
-  F.cs2[iel] = cs2;
   if (imx >= 0 && !learned) {
     const int c0 = F.imxfcp[imx], nc = F.imxncp[imx];
     for (int k = 0; k < nc; k++) {
@@ -2264,7 +2301,9 @@ void launch_lag_accel(const DevFields& F, const DevCfg& C, cudaStream_t s) {
   k_lag_accel<BS_ND, false><<<(F.nnd + BS_ND - 1) / BS_ND, BS_ND, 0, s>>>(F, C);
 }
 void launch_lag_state(const DevFields& F, const DevCfg& C, cudaStream_t s) {
-  k_lag_state<BS_EL, false><<<(F.nel + BS_EL - 1) / BS_EL, BS_EL, 0, s>>>(F, C);
+  const int g = (F.nel + BS_EL - 1) / BS_EL;
+  if (F.loop_ale) k_lag_state<BS_EL, false, true><<<g, BS_EL, 0, s>>>(F, C);
+  else k_lag_state<BS_EL, false><<<g, BS_EL, 0, s>>>(F, C);
 }
 constexpr size_t kClosureSmem = sizeof(mlp::SmemW) + kClosureWarps * sizeof(mlp::SmemS);
 int prepare_mix_closure() {
@@ -2308,7 +2347,9 @@ void launch_lag_accel_batch(const DevFields& F, const DevCfg& C, cudaStream_t s)
   else k_lag_accel<256, true><<<(F.nnd + 255) / 256, 256, 0, s>>>(F, C);
 }
 void launch_lag_state_batch(const DevFields& F, const DevCfg& C, cudaStream_t s) {
-  k_lag_state<BS_EL, true><<<(F.nel + BS_EL - 1) / BS_EL, BS_EL, 0, s>>>(F, C);
+  const int g = (F.nel + BS_EL - 1) / BS_EL;
+  if (F.loop_ale) k_lag_state<BS_EL, true, true><<<g, BS_EL, 0, s>>>(F, C);
+  else k_lag_state<BS_EL, true><<<g, BS_EL, 0, s>>>(F, C);
 }
 
 }  // namespace BL_NS
