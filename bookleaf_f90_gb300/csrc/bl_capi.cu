@@ -1615,7 +1615,7 @@ int bl_init_batch(bl_ctx** out, int ninst, const bl_sizes* sizes, const bl_confi
     I.el_begin = el_off[i];
     I.el_end = el_off[i + 1];
     I.blk_begin = nblk;
-    nblk += x->L.getdt_blocks(sizes[i].nel);
+    nblk += x->L.getdt_blocks(sizes[i].nel, S.nel);
     I.blk_end = nblk;
     for (int k = el_off[i]; k < el_off[i + 1]; k++) elinst[k] = i;
     for (int k = nd_off[i]; k < nd_off[i + 1]; k++) ndinst[k] = i;

@@ -14,7 +14,7 @@ namespace bl {
 
 #define BL_DECLARE_LAUNCHERS(NS)                                                   \
   namespace NS {                                                                   \
-  int getdt_blocks(int nel);                                                       \
+  int getdt_blocks(int nel, int all_nel);                                          \
   int getdt_grid(int nel);                                                         \
   void launch_getdt(const DevFields& F, const DevCfg& C, cudaStream_t s);          \
   void launch_lag_force(const DevFields& F, const DevCfg& C, cudaStream_t s);      \
@@ -37,7 +37,7 @@ BL_DECLARE_LAUNCHERS(exact)
 BL_DECLARE_LAUNCHERS(mixed)
 
 struct Launchers {
-  int (*getdt_blocks)(int);  // k_getdt blocks of one mesh in a batch
+  int (*getdt_blocks)(int, int);  // k_getdt blocks of one mesh of a batch (its elements, all)
   int (*getdt_grid)(int);    // k_getdt grid (and partials) of a single mesh
   void (*getdt)(const DevFields&, const DevCfg&, cudaStream_t);
   void (*lag_force)(const DevFields&, const DevCfg&, cudaStream_t);

@@ -273,19 +273,18 @@ __device__ __forceinline__ double min_dln(const double* x, const double* y, doub
   return m;
 }
 
-#if BL_FAST_ALGEBRA
-// Fast build: the same squared lengths from the element's iso-parametric
+#if BL_MIXED
+// Mixed build: the same squared lengths from the element's iso-parametric
 // coefficients.  For side k the opposite edge (corners k+2 -> k+3) is
 // 2*(dx,dy) with (dx,dy) = (a1+a2, b1+b2), (a2-a3, b2-b3), (a1-a2, b1-b2),
 // (a2+a3, b2+b3), and its cross product with the vector to the midpoint of
 // corners k,k+1 is 4*(dx*q - dy*p) with (p,q) = (a3,b3), (a1,b1), (a3,b3),
 // (a1,b1); so the reference's distpl/denom is 4 X^2 / Y with X = dx*q -
 // dy*p and Y = dx^2 + dy^2 (exact in real arithmetic), and its denominator
-// is 4 Y.  A degenerate opposite edge (4 Y < zcut) takes the corner form.
-// (T: FP64, or FP32 in the mixed build)
-template <class T>
-__device__ __forceinline__ T min_dln_iso(const double* x, const double* y, T zcut, T a1, T a2,
-                                         T a3, T b1, T b2, T b3) {
+// is 4 Y.  A degenerate opposite edge (4 Y < zcut) takes the corner form,
+// for which corners(x, y) then brings the positions.
+template <class T, class Q>
+__device__ __forceinline__ T min_dln_iso(Q corners, T zcut, T a1, T a2, T a3, T b1, T b2, T b3) {
   const T dxs[4] = {a1 + a2, a2 - a3, a1 - a2, a2 + a3};
   const T dys[4] = {b1 + b2, b2 - b3, b1 - b2, b2 + b3};
   T r[4];
@@ -296,6 +295,8 @@ __device__ __forceinline__ T min_dln_iso(const double* x, const double* y, T zcu
     const T Y = dx * dx + dy * dy;
     if (gt_nn(zcut, times4(Y))) {
       const int a = k, b = (k + 1) & 3, c = (k + 2) & 3;
+      double x[4], y[4];
+      corners(x, y);
       r[k] = (T)g_distpp(x[a], y[a], x[b], y[b], x[c], y[c]);
     } else {
       const T X = dx * q - dy * p;
@@ -523,17 +524,22 @@ struct DevLayout {
 // The element's squared CFL length of hydro_kn_getdtcfl (min over its
 // sides of geometry_kn_dlm or _dln), or -1 for a zdtnotreg region (the
 // reference's HUGE candidate); it does not depend on the viscosity.
-template <class L = DevLayout>
+// corners(x, y) brings the corner positions where they are needed.
+template <class L = DevLayout, class Q>
 __device__ __forceinline__ double getdt_cfl_len(const DevFields& F, const DevCfg& C, int iel,
-                                                const double* x, const double* y) {
+                                                Q corners) {
   const int ireg = L::reg(F, iel);
   if (__ldg(C.zdtnotreg + ireg)) return -1.0;
-#if BL_FAST_ALGEBRA
-  return __ldg(C.zmidlength + ireg)
-             ? min_dlm(x, y)
-             : from_lr(min_dln_iso<lr>(x, y, lr_cut(C.zcut), to_lr(F.a1[iel]), to_lr(F.a2[iel]),
-                                       to_lr(F.a3[iel]), to_lr(F.b1[iel]), to_lr(F.b2[iel]),
-                                       to_lr(F.b3[iel])));
+#if BL_MIXED
+  if (!__ldg(C.zmidlength + ireg))
+    return from_lr(min_dln_iso<lr>(corners, lr_cut(C.zcut), to_lr(F.a1[iel]), to_lr(F.a2[iel]),
+                                   to_lr(F.a3[iel]), to_lr(F.b1[iel]), to_lr(F.b2[iel]),
+                                   to_lr(F.b3[iel])));
+#endif
+  double x[4], y[4];
+  corners(x, y);
+#if BL_MIXED
+  return min_dlm(x, y);
 #else
   return __ldg(C.zmidlength + ireg) ? min_dlm(x, y) : min_dln(x, y, C.zcut);
 #endif
@@ -594,12 +600,12 @@ __device__ __forceinline__ void getdt_cfl(const DevFields& F, int iel, double le
 
 // hydro_dr_getcs2, then the element's hydro_kn_getdtcfl and getdtdiv
 // candidates
-template <class L = DevLayout>
+template <class L = DevLayout, class Q>
 __device__ __forceinline__ void getdt_tail(const DevFields& F, const DevCfg& C, int iel,
-                                           const double* x, const double* y, const double* u,
-                                           const double* v, double visc, double& cflv, int& cfli,
-                                           double& divv, int& divi) {
-  getdt_cfl(F, iel, getdt_cfl_len<L>(F, C, iel, x, y), visc, cflv, cfli);
+                                           Q corners, const double* u, const double* v,
+                                           double visc, double& cflv, int& cfli, double& divv,
+                                           int& divi) {
+  getdt_cfl(F, iel, getdt_cfl_len<L>(F, C, iel, corners), visc, cflv, cfli);
   getdt_div(F, iel, u, v, divv, divi);
 }
 
@@ -798,6 +804,21 @@ __device__ __forceinline__ void getdt_finish(const DevFields& F, const DevCfg& C
   }
 }
 
+// Consecutive tiles of BS elements that a k_getdt block of the fast and mixed
+// builds takes, for nel elements in all meshes together: about as many blocks
+// as are resident at once (152 SMs of 7), at least one tile and at most 8.  A
+// block ends with a barrier and a ticket of a microsecond, which 8,192 blocks
+// of one tile each pay one after another on every SM: Noh 1024x1024, 1, 2, 4,
+// 8 and 16 tiles, the mixed build's k_edgevisc + k_getdt 203, 190, 180, 172,
+// 196 us, the fast build's pair 261, 259, 258, 259, 280; Sedov 512x512 (2,048
+// tiles) 1, 2 and 4 tiles 65.3, 63.6, 67.6 us; fewer than 1.5 tiles a resident
+// block are better left one each.
+__host__ __device__ __forceinline__ int getdt_tiles(int nel, int bs) {
+  if (!BL_FAST_ALGEBRA) return 1;
+  const int t = (nel / bs + 532) / 1064;
+  return t < 1 ? 1 : (t > 8 ? 8 : t);
+}
+
 #if BL_FAST_ALGEBRA
 // The quantities of a face that both elements sharing it compute -- its
 // lengths, unit vectors and the inverse ratio of its projections -- from
@@ -839,7 +860,10 @@ __device__ __forceinline__ lr nb_ratio(const FaceQ& f, lr ddx, lr ddy, lr ddu, l
 #endif
 }
 #if BL_MIXED
-// k_getdt of the mixed build shares face work between neighbouring threads.
+// ================================================================ k_edgevisc
+
+// The mixed build's edge viscosity (elvisc and the corner forces); k_getdt
+// reads elvisc back.  It shares face work between neighbouring threads.
 // A block of BS threads takes BS - 2 consecutive elements; thread t holds
 // element blockIdx*(BS-2) + t - 1, so threads 0 and BS-1 hold the
 // neighbours of the block's first and last elements (halos).  Every
@@ -855,43 +879,20 @@ __device__ __forceinline__ lr nb_ratio(const FaceQ& f, lr ddx, lr ddy, lr ddu, l
 // generated meshes elements are numbered along mesh lines, so the face
 // across face 2 and the two limiter neighbours of side 0 are the adjacent
 // elements and take the shared path.
-// Launched twice: PART 1, the edge viscosity (elvisc and the corner
-// forces), then PART 2, which reads elvisc back for the CFL and divergence
-// candidates and the dt reduction (the same blocks over the same elements
-// in both); neither half spills, and the pair takes 62.1 us on Sedov
-// 512x512 against 68.7-71.0 us in one kernel.  The FP64 build's form, one
-// thread per edge of the mesh (k_edge), would take 59 us here, but FP32
-// rounds each of an edge's two sides its own way: it would change results
-// in the seventh digit, so the element form stays.
-template <int BS, bool BATCH, int PART>
-__global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg C) {
-  // the mesh of this block: the context's, or in a batch the block's own
-  // (its blocks [blk0, blk0 + nblk), elements [el0, el1))
-  DevStep* S = F.step;
-  int blk0 = 0, nblk = (int)gridDim.x, el0 = 0, el1 = F.nel;
-  const DevInst* I = nullptr;
-  if (BATCH) {
-    const int m = __ldg(F.blkinst + blockIdx.x);
-    I = F.inst + m;
-    S = F.steps + m;
-    blk0 = I->blk_begin;
-    nblk = I->blk_end - I->blk_begin;
-    el0 = I->el_begin;
-    el1 = I->el_end;
-  }
-  if (halted(S)) return;
-  if (S->stop_next) {            // bl_run: the previous step reached time_end
-    if ((int)blockIdx.x == blk0 && threadIdx.x == 0) S->halted = 1;
-    return;
-  }
+// The FP64 build's form, one thread per edge of the mesh (k_edge), would be
+// no slower here, but FP32 rounds each of an edge's two sides its own way: it
+// would change results in the seventh digit, so the element form stays.
+template <int BS, bool BATCH>
+__global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_edgevisc(DevFields F, DevCfg C) {
   const int t = threadIdx.x;
-  const int iel = el0 + ((int)blockIdx.x - blk0) * (BS - 2) + t - 1;
-  const bool inmesh = iel >= el0 && iel < el1;
+  const int iel = (int)blockIdx.x * (BS - 2) + t - 1;
+  if (!BATCH && (halted(F.step) || F.step->stop_next)) return;
+  bool inmesh = iel >= 0 && iel < F.nel;
+  if (BATCH && inmesh) {
+    const DevStep* S = el_step<true>(F, iel);
+    inmesh = !(halted(S) || S->stop_next);
+  }
   const bool own = inmesh && t > 0 && t < BS - 1;
-  double cflv = HUGE_VAL;        // sentinel above HUGE(1.0)
-  int cfli = 0x7fffffff;
-  double divv = DBL_MIN;         // TINY(1.0)
-  int divi = -1;
   // face 0: du dv lu lx uh vh xh yh w1, then the edge coefficient's two
   // factors that do not depend on the side the face is seen from,
   // cvisc1*sqrt((cs2 + cs2')/2) + cvisc2*|du| and rho + rho' (the same sums
@@ -915,7 +916,7 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
       v[j] = F.ndv[n[j]];
     }
   }
-  if (PART != 2 && !C.ztq) {
+  {
     if (inmesh) {
       const FaceQ f0 = face_q(to_lr(u[1] - u[0]), to_lr(v[1] - v[0]), to_lr(x[1] - x[0]),
                               to_lr(y[1] - y[0]), zl);
@@ -944,8 +945,7 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
   }
   if (own) {
     const double rho0 = F.rho[iel];
-    double visc = 0.0;
-    if (PART != 2 && !C.ztq) {
+    {
       // hydro_kn_initeviscosity / limiteviscosity / geteviscosity
       // (hydro_kn_edgeviscosity.f90:30-282), face by face in the reference's
       // order 3, 1, 0, 2 (the faces of side s are (s+3)&3 and s+1)
@@ -1079,22 +1079,70 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
           }
         }
       }
-      visc = from_lr(vmax * DIV((lr)2, maxF(to_lr(rho0), zl)));
+      const double visc = from_lr(vmax * DIV((lr)2, maxF(to_lr(rho0), zl)));
       F.cnviscx[iel] = make_d4(from_lr(edx[0] - edx[3]), from_lr(edx[1] - edx[0]),
                                from_lr(edx[2] - edx[1]), from_lr(edx[3] - edx[2]));
       F.cnviscy[iel] = make_d4(from_lr(edy[0] - edy[3]), from_lr(edy[1] - edy[0]),
                                from_lr(edy[2] - edy[1]), from_lr(edy[3] - edy[2]));
       F.visc[iel] = visc;
-    } else {
-      visc = F.visc[iel];
     }
-    if (PART != 1) getdt_tail(F, C, iel, x, y, u, v, visc, cflv, cfli, divv, divi);
   }
-  if (PART != 1) getdt_finish<BS, BATCH>(F, C, S, cflv, cfli, divv, divi, blk0, nblk, el0, I);
 }
 
-template <int BS>
-constexpr int getdt_elements_per_block() { return BS - 2; }
+// ================================================================ k_getdt
+
+// The mixed build's CFL and divergence candidates and the dt reduction, one
+// thread per element.  Bound by its loads' latency (4 FP64 instructions an
+// element): the positions are brought only for the regions and faces that
+// need them, and a block takes several tiles.  (8, 10 and 12 blocks per SM,
+// with the registers that leaves, are slower.)
+template <int BS, bool BATCH>
+__global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg C) {
+  DevStep* S = F.step;
+  int blk0 = 0, nblk = (int)gridDim.x, el0 = 0, el1 = F.nel;
+  const DevInst* I = nullptr;
+  if (BATCH) {
+    const int m = __ldg(F.blkinst + blockIdx.x);
+    I = F.inst + m;
+    S = F.steps + m;
+    blk0 = I->blk_begin;
+    nblk = I->blk_end - I->blk_begin;
+    el0 = I->el_begin;
+    el1 = I->el_end;
+  }
+  if (halted(S)) return;
+  if (S->stop_next) {            // bl_run: the previous step reached time_end
+    if ((int)blockIdx.x == blk0 && threadIdx.x == 0) S->halted = 1;
+    return;
+  }
+  double cflv = HUGE_VAL;        // sentinel above HUGE(1.0)
+  int cfli = 0x7fffffff;
+  double divv = DBL_MIN;         // TINY(1.0)
+  int divi = -1;
+  const int tiles = getdt_tiles(F.nel, BS);
+  int iel = el0 + ((int)blockIdx.x - blk0) * tiles * BS + (int)threadIdx.x;
+  for (int k = 0; k < tiles && iel < el1; k++, iel += BS) {
+    const int4 nd = __ldg(F.ielnd + iel);
+    const int n[4] = {nd.x, nd.y, nd.z, nd.w};
+    double u[4], v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      u[j] = F.ndu[n[j]];
+      v[j] = F.ndv[n[j]];
+    }
+    auto corners = [&](double* x, double* y) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        x[j] = F.ndx[n[j]];
+        y[j] = F.ndy[n[j]];
+      }
+    };
+    getdt_tail(F, C, iel, corners, u, v, F.visc[iel], cflv, cfli, divv, divi);
+  }
+  getdt_finish<BS, BATCH>(F, C, S, cflv, cfli, divv, divi, blk0, nblk, el0, I);
+}
+
+
 #else
 // Two kernels.  k_edge computes every edge of the mesh once
 // (bl_setup.cuh: its slots); k_getdt then takes each element's four edges
@@ -1339,8 +1387,9 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
     el0 = I->el_begin;
     el1 = I->el_end;
   }
-  const int iel = el0 + ((int)blockIdx.x - blk0) * BS + (int)threadIdx.x;
-  // (the tables' loads leave before the header's answer is needed)
+  const int tiles = getdt_tiles(F.nel, BS);
+  int iel = el0 + ((int)blockIdx.x - blk0) * tiles * BS + (int)threadIdx.x;
+  // (the table's load leaves before the header's answer is needed)
   uint4 er4 = make_uint4(0u, 0u, 0u, 0u);
   if (iel < el1) er4 = __ldg(F.eref + iel);
   if (halted(S)) return;
@@ -1352,7 +1401,8 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
   int cfli = 0x7fffffff;
   double divv = DBL_MIN;         // TINY(1.0)
   int divi = -1;
-  if (iel < el1) {
+  for (int k = 0; k < tiles && iel < el1; k++, iel += BS) {
+    if (k > 0) er4 = __ldg(F.eref + iel);
     const unsigned er[4] = {er4.x, er4.y, er4.z, er4.w};
     double visc = 0.0;
     double du[4], dv[4], sq[4], W[4], edx[4], edy[4];
@@ -1405,8 +1455,8 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
       visc = F.visc[iel];
     }
     const double cs2v = signal_speed(F, iel, cs2, visc);
-    cflv = cfl_candidate(F, C, iel, W, sq, a1, a2, a3, b1, b2, b3, cs2v, notdt, mid);
-    cfli = iel;
+    cfl_min(cflv, cfli, cfl_candidate(F, C, iel, W, sq, a1, a2, a3, b1, b2, b3, cs2v, notdt, mid),
+            iel);
     const double w = b1 * (du[3] - du[1]) + b3 * (du[0] - du[2]) - a1 * (dv[3] - dv[1]) -
                      a3 * (dv[0] - dv[2]);
     const double dd = DIV(absF(w), vol);
@@ -1418,8 +1468,6 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
   getdt_finish<BS, BATCH>(F, C, S, cflv, cfli, divv, divi, blk0, nblk, el0, I);
 }
 
-template <int BS>
-constexpr int getdt_elements_per_block() { return BS; }
 #endif
 #else
 
@@ -1589,13 +1637,18 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
     } else {
       visc = F.visc[iel];
     }
-    getdt_tail<L>(F, C, iel, x, y, u, v, visc, cflv, cfli, divv, divi);
+    auto corners = [&](double* cx, double* cy) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        cx[j] = x[j];
+        cy[j] = y[j];
+      }
+    };
+    getdt_tail<L>(F, C, iel, corners, u, v, visc, cflv, cfli, divv, divi);
   }
   getdt_finish<BS, BATCH>(F, C, S, cflv, cfli, divv, divi, blk0, nblk, el0, I);
 }
 
-template <int BS>
-constexpr int getdt_elements_per_block() { return BS; }
 #endif
 
 // ================================================================ k_lag_force
@@ -2261,19 +2314,18 @@ static constexpr int BS_EL = 128;
 static constexpr int BS_ED = 128;  // k_edge
 static constexpr int BS_ND = 128;
 
-// one block per getdt_elements_per_block elements
-int getdt_blocks(int nel) {
-  constexpr int E = getdt_elements_per_block<BS_DT>();
-  return (nel + E - 1) / E;
+// k_getdt blocks of a mesh of nel elements, of all_nel in the context
+int getdt_blocks(int nel, int all_nel) {
+  const int per = BS_DT * getdt_tiles(all_nel, BS_DT);
+  return (nel + per - 1) / per;
 }
 
-// a single mesh's grid and number of partials: the same blocks (an equal
-// share per block over whole resident waves was measured slower: the SMs'
-// spread of finishing times is a spread of their speeds, not of their work)
-int getdt_grid(int nel) { return getdt_blocks(nel); }
+// a single mesh's grid and number of partials
+int getdt_grid(int nel) { return getdt_blocks(nel, nel); }
 
-// k_edge: BS_ED - 2 slots a block
-[[maybe_unused]] static int edge_grid(int nslot) { return (nslot + BS_ED - 3) / (BS_ED - 2); }
+// k_edge, k_edgevisc: BS - 2 slots or elements a block
+static_assert(BS_ED == BS_DT, "one edge_grid");
+[[maybe_unused]] static int edge_grid(int n) { return (n + BS_ED - 3) / (BS_ED - 2); }
 
 int getdt_launches(const DevCfg& C) {
 #if BL_MIXED
@@ -2285,14 +2337,11 @@ int getdt_launches(const DevCfg& C) {
 }
 void launch_getdt(const DevFields& F, const DevCfg& C, cudaStream_t s) {
 #if BL_MIXED
-  if (!C.ztq) k_getdt<BS_DT, false, 1><<<getdt_grid(F.nel), BS_DT, 0, s>>>(F, C);
-  k_getdt<BS_DT, false, 2><<<getdt_grid(F.nel), BS_DT, 0, s>>>(F, C);
-#else
-#if BL_FAST_ALGEBRA
+  if (!C.ztq) k_edgevisc<BS_DT, false><<<edge_grid(F.nel), BS_DT, 0, s>>>(F, C);
+#elif BL_FAST_ALGEBRA
   k_edge<BS_ED, false><<<edge_grid(F.nslot), BS_ED, 0, s>>>(F, C);
 #endif
   k_getdt<BS_DT, false><<<getdt_grid(F.nel), BS_DT, 0, s>>>(F, C);
-#endif
 }
 void launch_lag_force(const DevFields& F, const DevCfg& C, cudaStream_t s) {
   k_lag_force<BS_EL, false><<<(F.nel + BS_EL - 1) / BS_EL, BS_EL, 0, s>>>(F, C);
@@ -2328,14 +2377,11 @@ void launch_mix_closure_batch(const DevFields& F, const DevCfg& C, cudaStream_t 
 // elements or nodes, each reading the step header of its mesh
 void launch_getdt_batch(const DevFields& F, const DevCfg& C, cudaStream_t s) {
 #if BL_MIXED
-  if (!C.ztq) k_getdt<BS_DT, true, 1><<<F.nblk_batch, BS_DT, 0, s>>>(F, C);
-  k_getdt<BS_DT, true, 2><<<F.nblk_batch, BS_DT, 0, s>>>(F, C);
-#else
-#if BL_FAST_ALGEBRA
+  if (!C.ztq) k_edgevisc<BS_DT, true><<<edge_grid(F.nel), BS_DT, 0, s>>>(F, C);
+#elif BL_FAST_ALGEBRA
   k_edge<BS_ED, true><<<edge_grid(F.nslot), BS_ED, 0, s>>>(F, C);
 #endif
   k_getdt<BS_DT, true><<<F.nblk_batch, BS_DT, 0, s>>>(F, C);
-#endif
 }
 void launch_lag_force_batch(const DevFields& F, const DevCfg& C, cudaStream_t s) {
   k_lag_force<BS_EL, true><<<(F.nel + BS_EL - 1) / BS_EL, BS_EL, 0, s>>>(F, C);
