@@ -6,8 +6,8 @@
 // bl_getdt's computation (edge viscosity, elcs2+elvisc, CFL and divergence
 // limits, dt selection) on device arrays the caller passes, in the
 // reference's own layout, without a bl_ctx.  It launches the library's own
-// exact-form k_getdt (hydro_kernels.cuh, compiled here like the exact
-// build, without FMA contraction), reading the caller's 1-based (NCORN,nel)
+// exact-form k_edge and k_getdt (hydro_kernels.cuh, compiled here like the
+// exact build, without FMA contraction), reading the caller's 1-based (NCORN,nel)
 // connectivity through RefLayout below; its results equal bl_getdt's in
 // BL_FP_EXACT mode bit for bit.
 //
@@ -63,13 +63,6 @@ struct RefLayout {
   static __device__ __forceinline__ int reg(const bl::DevFields& F, int e) {
     const int r = __ldg(F.ielreg + e) - 1;
     return (r < 0 || r >= BL_MAXREG) ? 0 : r;
-  }
-  static __device__ __forceinline__ void corners(bl::d4* p, int e, const double* q) {
-    double* o = reinterpret_cast<double*>(p) + 4 * (size_t)e;
-    o[0] = q[0];
-    o[1] = q[1];
-    o[2] = q[2];
-    o[3] = q[3];
   }
 };
 
@@ -227,6 +220,7 @@ extern "C" int bl_getdt_noalloc(const bl_getdt_arrays* arrays, const bl_config* 
     return BL_FAILURE;
   }
   const int blocks = (A.nel + kBS - 1) / kBS;
+  if (!C.ztq) bl::na::k_edge<kBS, false, RefLayout><<<(A.nel + kBS / 4 - 1) / (kBS / 4), kBS, 0, s>>>(F, C);
   bl::na::k_getdt<kBS, false, RefLayout><<<blocks, kBS, 0, s>>>(F, C);
   bl::DevStep R;
   r = cudaGetLastError();

@@ -496,13 +496,10 @@ __device__ __forceinline__ void div_max(double& v, int& i, double ov, int oi) {
   if (io > iv || (io == iv && oi >= 0 && (i < 0 || oi < i))) { v = ov; i = oi; }
 }
 
-// hydro_dr_getcs2 (elcs2 += elvisc; mixed cells: sum frmass*(cpcs2+cpvisc)),
-// then the element's hydro_kn_getdtcfl and getdtdiv candidates
-// How k_getdt reads an element's connectivity and region and stores its
-// corner forces: in the library's own layout (0-based rows of four, face
-// numbers packed in one int, 32-byte corner vectors).  The exact-form
-// kernel takes the layout as a parameter, so that bl_getdt_noalloc runs the
-// same kernel on arrays in the reference's layout.
+// How the getdt kernels read an element's connectivity and region: in the
+// library's own layout (0-based rows of four, face numbers packed in one
+// int).  The exact-form kernels take the layout as a parameter, so that
+// bl_getdt_noalloc runs the same kernels on arrays in the reference's layout.
 struct DevLayout {
   static __device__ __forceinline__ int4 nodes(const DevFields& F, int e) {
     return __ldg(F.ielnd + e);
@@ -515,9 +512,6 @@ struct DevLayout {
   }
   static __device__ __forceinline__ int reg(const DevFields& F, int e) {
     return __ldg(F.ielreg + e);
-  }
-  static __device__ __forceinline__ void corners(d4* p, int e, const double* q) {
-    p[e] = make_d4(q[0], q[1], q[2], q[3]);
   }
 };
 
@@ -1471,6 +1465,136 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
 #endif
 #else
 
+// ================================================================ k_edge
+
+// Exact build: the edge viscosity, one thread per face of an element, four
+// adjacent threads an element.  Both elements of an edge compute it, each in
+// its own order (a reversed difference can differ from the recomputed one in
+// the sign of a zero), and every expression is the reference's; the quad
+// joins its faces through shuffles.  One thread per element took its four
+// faces one after another with 676 bytes of spills; the step of a 1,000-element
+// tube took 66.9 us, now 41.6, Sedov 128x128 89.8, now 68.5, 512x512 596, now 581.
+#ifndef BL_EDGE_MINB
+#define BL_EDGE_MINB 7
+#endif
+template <int BS, bool BATCH, class L = DevLayout>
+__global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C) {
+  const long long at = (long long)blockIdx.x * BS + threadIdx.x;
+  const int iel = (int)(at >> 2), is = (int)(at & 3), jn = (is + 1) & 3;
+  bool in = iel < F.nel;  // the same for a quad
+  if (!BATCH && (halted(F.step) || F.step->stop_next)) return;
+  if (BATCH && in) {
+    const DevStep* S = el_step<true>(F, iel);
+    in = !(halted(S) || S->stop_next);
+  }
+  double ex = 0.0, ey = 0.0, visc = 0.0;
+  if (in) {
+    // hydro_kn_initeviscosity / limiteviscosity / geteviscosity
+    // (hydro_kn_edgeviscosity.f90:30-282).  Face is runs corner is -> is+1;
+    // the faces of side s (neighbours across faces s and s+2) are (s+3)&3
+    // and s+1.
+    const int4 n = L::nodes(F, iel), nb = L::nbrs(F, iel);
+    const int fcp = L::faces(F, iel);
+    const double zc = C.zerocut;
+    const double rho0 = F.rho[iel], cs2i = F.cs2[iel];
+    const double x[4] = {F.ndx[n.x], F.ndx[n.y], F.ndx[n.z], F.ndx[n.w]};
+    const double y[4] = {F.ndy[n.x], F.ndy[n.y], F.ndy[n.z], F.ndy[n.w]};
+    const double xc = quarter(x[0] + x[1] + x[2] + x[3]);
+    const double yc = quarter(y[0] + y[1] + y[2] + y[3]);
+    auto pick = [](const double* v, int j) {
+      return j == 0 ? v[0] : (j == 1 ? v[1] : (j == 2 ? v[2] : v[3]));
+    };
+    auto ipick = [](const int4& v, int j) {
+      return j == 0 ? v.x : (j == 1 ? v.y : (j == 2 ? v.z : v.w));
+    };
+    const double xa = pick(x, is), xb = pick(x, jn), ya = pick(y, is), yb = pick(y, jn);
+    const int na = ipick(n, is), nn = ipick(n, jn);
+    const int s = (is & 1) ? 0 : 1;
+    const bool first = is == 3 || is == 0;
+    const int in1 = ipick(nb, s), in2 = ipick(nb, s + 2);
+    const int f1 = fc_of(fcp, s), f2 = fc_of(fcp, s + 2);
+    // boundary rule (hydro_kn_edgeviscosity.f90:154-183): a ratio across a
+    // boundary face is 1 between two boundary nodes facing an interior
+    // neighbour, 0 otherwise
+    double r1 = 0.0, r2 = 0.0;
+    if (in1 == iel)
+      r1 = (__ldg(F.indtype + ipick(n, s)) < 0 && __ldg(F.indtype + ipick(n, s + 1)) < 0 &&
+            in2 != iel) ? 1.0 : 0.0;
+    if (in2 == iel)
+      r2 = (__ldg(F.indtype + ipick(n, s + 2)) < 0 &&
+            __ldg(F.indtype + ipick(n, (s + 3) & 3)) < 0 && in1 != iel) ? 1.0 : 0.0;
+    double w1 = F.ndu[nn] - F.ndu[na], w2 = F.ndv[nn] - F.ndv[na];
+    double w3 = xb - xa, w4 = yb - ya;
+    const double du = w1, dv = w2;
+    double den = SQRT(w1 * w1 + w2 * w2);
+    const double lu = den;
+    den = DIV(1.0, maxF_nn(den, zc));
+    const double uhat = w1 * den, vhat = w2 * den;
+    den = SQRT(w3 * w3 + w4 * w4);
+    const double lx = den;
+    den = DIV(1.0, maxF_nn(den, zc));
+    const double xh = w3 * den, yh = w4 * den;
+    den = w3 * xh + w4 * yh;
+    w1 = DIV(w1 * uhat + w2 * vhat, signF(maxF_nn(absF(den), zc), den));
+    w1 = DIV(1.0, signF(maxF_nn(absF(w1), zc), w1));
+    // neighbour faces: edge 1 uses MOD(ielfc,4)+1 / MOD(ielfc+2,4)+1,
+    // edge 2 the other pair (hydro_kn_edgeviscosity.f90:117-151)
+    auto ratio = [&](int nbr, int face) {
+      const int4 m = L::nodes(F, nbr);
+      const int a = ipick(m, face), b = ipick(m, (face + 1) & 3);
+      const double ddx = F.ndx[b] - F.ndx[a], ddy = F.ndy[b] - F.ndy[a];
+      const double ddu = F.ndu[b] - F.ndu[a], ddv = F.ndv[b] - F.ndv[a];
+      const double dn = ddx * xh + ddy * yh;
+      const double q = DIV(ddu * uhat + ddv * vhat, signF(maxF_nn(absF(dn), zc), dn));
+      return q * w1;
+    };
+    if (in1 != iel) r1 = ratio(in1, (f1 + (first ? 1 : 3)) & 3);
+    if (in2 != iel) r2 = ratio(in2, (f2 + (first ? 3 : 1)) & 3);
+    // limiter and edge coefficient (hydro_kn_edgeviscosity.f90:185-214)
+    const int ins = ipick(nb, is);
+    w1 = C.cvisc1 * SQRT(half(cs2i + F.cs2[ins]));
+    w2 = minF(minF(minF(half(r1 + r2), twice(r1)), twice(r2)), 1.0);
+    w2 = maxF(0.0, w2);
+    w3 = half(1.0 - w2) * (rho0 + F.rho[ins]) * (w1 + C.cvisc2 * lu);
+    const double edv = w3;
+    visc = maxF_nn(0.0, w3 * DIV(twice(lu), maxF(rho0, zc)));
+    // edge force (hydro_kn_edgeviscosity.f90:219-282)
+    const double m3 = half(xa + xb);
+    const double m6 = half(ya + yb);
+    const double w7 = SQRT((xc - m3) * (xc - m3) + (yc - m6) * (yc - m6));
+    double d = DIV(1.0, w7);
+    double exh = (yc - m6) * d, eyh = (m3 - xc) * d;
+    // w1*(1/w8), w4*(1/w8) with w8 the face's length: the limiter's
+    // normalised face vector whenever w8 > zerocut; otherwise the edge is
+    // cut below
+    const double w33 = exh * xh + eyh * yh;
+    d = -(signF(1.0, w33) * w7);
+    exh = exh * d;
+    eyh = eyh * d;
+    const double w6b = du * exh + dv * eyh;
+    d = DIV(w6b, maxF_nn(lu, zc));
+    if (!(le_nn(lu, zc) || geF(zc, w6b) || le_nn(w7, zc) || le_nn(lx, zc))) {
+      ex = edv * du * d;
+      ey = edv * dv * d;
+    }
+  }
+  // corner j's force is the difference of faces j and j - 1; elvisc is the
+  // largest of the four faces' (never negative: +0 or positive)
+  const int from = (threadIdx.x & 28) | ((is + 3) & 3);
+  const double px = __shfl_sync(0xffffffffu, ex, from), py = __shfl_sync(0xffffffffu, ey, from);
+  visc = maxF_nn(visc, __shfl_xor_sync(0xffffffffu, visc, 1));
+  visc = maxF_nn(visc, __shfl_xor_sync(0xffffffffu, visc, 2));
+  if (in) {
+    reinterpret_cast<double*>(F.cnviscx)[at] = ex - px;
+    reinterpret_cast<double*>(F.cnviscy)[at] = ey - py;
+    if (is == 0) F.visc[iel] = visc;
+  }
+}
+
+// ================================================================ k_getdt
+
+// Exact build: hydro_dr_getcs2, the CFL and divergence candidates and the dt
+// reduction, after k_edge.
 template <int BS, bool BATCH, class L = DevLayout>
 __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg C) {
   // the mesh of this block: the context's, or in a batch the block's own
@@ -1500,155 +1624,23 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
   if (iel < el1) {
     const int4 nd = L::nodes(F, iel);
     const int n[4] = {nd.x, nd.y, nd.z, nd.w};
-    double x[4], y[4], u[4], v[4];
+    double u[4], v[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      x[j] = F.ndx[n[j]];
-      y[j] = F.ndy[n[j]];
       u[j] = F.ndu[n[j]];
       v[j] = F.ndv[n[j]];
     }
-    const double zc = C.zerocut;
-    const double rho0 = F.rho[iel];
-    double visc = 0.0;
-    double qx[4] = {0.0, 0.0, 0.0, 0.0}, qy[4] = {0.0, 0.0, 0.0, 0.0};
-    if (!C.ztq) {
-      // hydro_kn_initeviscosity / limiteviscosity / geteviscosity
-      // (hydro_kn_edgeviscosity.f90:30-282), evaluated face by face: every
-      // quantity of a face -- its differences (face j runs corner j ->
-      // j+1), lengths, normalised vectors, limiter ratios, edge coefficient
-      // and edge force -- is formed and consumed before the next face, which
-      // keeps the live state to the element's corners and the four edge
-      // forces.  The faces of side s (neighbours across faces s and s+2)
-      // are (s+3)&3 and s+1, in the reference's order 3, 1, 0, 2.
-      const int4 ee = L::nbrs(F, iel);
-      const int nb[4] = {ee.x, ee.y, ee.z, ee.w};
-      const int fcp = L::faces(F, iel);
-      const double cs2i = F.cs2[iel];
-      const double xc = quarter(x[0] + x[1] + x[2] + x[3]);
-      const double yc = quarter(y[0] + y[1] + y[2] + y[3]);
-      double edx[4], edy[4];
-#pragma unroll
-      for (int s = 0; s < 2; s++) {
-        const int in1 = nb[s], in2 = nb[s + 2];
-        const int f1 = fc_of(fcp, s), f2 = fc_of(fcp, s + 2);
-        // boundary rule (hydro_kn_edgeviscosity.f90:154-183): a ratio across
-        // a boundary face is 1 between two boundary nodes facing an
-        // interior neighbour, 0 otherwise
-        double val1 = 0.0, val2 = 0.0;
-        if (in1 == iel)
-          val1 = (__ldg(F.indtype + n[s]) < 0 && __ldg(F.indtype + n[(s + 1) & 3]) < 0 && in2 != iel)
-                     ? 1.0 : 0.0;
-        if (in2 == iel)
-          val2 = (__ldg(F.indtype + n[s + 2]) < 0 && __ldg(F.indtype + n[(s + 3) & 3]) < 0 &&
-                  in1 != iel) ? 1.0 : 0.0;
-#pragma unroll
-        for (int e2 = 0; e2 < 2; e2++) {
-          const int is = e2 == 0 ? ((s + 3) & 3) : (s + 1);
-          const int jn = (is + 1) & 3;
-          double w1 = u[jn] - u[is], w2 = v[jn] - v[is];
-          double w3 = x[jn] - x[is], w4 = y[jn] - y[is];
-          const double du = w1, dv = w2;
-          double den = SQRT(w1 * w1 + w2 * w2);
-          const double lu = den;
-          den = DIV(1.0, maxF_nn(den, zc));
-          const double uhat = w1 * den, vhat = w2 * den;
-          den = SQRT(w3 * w3 + w4 * w4);
-          const double lx = den;
-          den = DIV(1.0, maxF_nn(den, zc));
-          const double xh = w3 * den, yh = w4 * den;
-          den = w3 * xh + w4 * yh;
-          w1 = DIV(w1 * uhat + w2 * vhat, signF(maxF_nn(absF(den), zc), den));
-          w1 = DIV(1.0, signF(maxF_nn(absF(w1), zc), w1));
-          // neighbour faces: edge 1 uses MOD(ielfc,4)+1 / MOD(ielfc+2,4)+1,
-          // edge 2 the other pair (hydro_kn_edgeviscosity.f90:117-151)
-          const int ins1 = e2 == 0 ? ((f1 + 1) & 3) : ((f1 + 3) & 3);
-          const int ins2 = e2 == 0 ? ((f2 + 3) & 3) : ((f2 + 1) & 3);
-          double r1 = val1, r2 = val2;
-          if (in1 != iel) {
-            const int4 m = L::nodes(F, in1);
-            const int mm[4] = {m.x, m.y, m.z, m.w};
-            const int a = mm[ins1], b = mm[(ins1 + 1) & 3];
-            double ddx = F.ndx[b] - F.ndx[a], ddy = F.ndy[b] - F.ndy[a];
-            double ddu = F.ndu[b] - F.ndu[a], ddv = F.ndv[b] - F.ndv[a];
-            double dn = ddx * xh + ddy * yh;
-            double q = DIV(ddu * uhat + ddv * vhat, signF(maxF_nn(absF(dn), zc), dn));
-            r1 = q * w1;
-          }
-          if (in2 != iel) {
-            const int4 m = L::nodes(F, in2);
-            const int mm[4] = {m.x, m.y, m.z, m.w};
-            const int a = mm[ins2], b = mm[(ins2 + 1) & 3];
-            double ddx = F.ndx[b] - F.ndx[a], ddy = F.ndy[b] - F.ndy[a];
-            double ddu = F.ndu[b] - F.ndu[a], ddv = F.ndv[b] - F.ndv[a];
-            double dn = ddx * xh + ddy * yh;
-            double q = DIV(ddu * uhat + ddv * vhat, signF(maxF_nn(absF(dn), zc), dn));
-            r2 = q * w1;
-          }
-          // limiter and edge coefficient (hydro_kn_edgeviscosity.f90:185-214)
-          const int ins = nb[is];
-          w1 = C.cvisc1 * SQRT(half(cs2i + F.cs2[ins]));
-          w2 = r1;
-          w3 = r2;
-          w2 = minF(minF(minF(half(w2 + w3), twice(w2)), twice(w3)), 1.0);
-          w2 = maxF(0.0, w2);
-          w4 = lu;
-          w3 = half(1.0 - w2) * (rho0 + F.rho[ins]) * (w1 + C.cvisc2 * w4);
-          const double edv = w3;
-          w4 = DIV(twice(w4), maxF(rho0, zc));
-          visc = maxF_nn(visc, w3 * w4);  // visc stays +0 or positive
-          // edge force (hydro_kn_edgeviscosity.f90:219-282)
-          {
-            const double m3 = half(x[is] + x[jn]);
-            const double m6 = half(y[is] + y[jn]);
-            const double w7 = SQRT((xc - m3) * (xc - m3) + (yc - m6) * (yc - m6));
-            const double w8 = lx;  // SQRT(w1*w1+w4*w4) of the same face difference
-            double d = DIV(1.0, w7);
-            double exh = (yc - m6) * d, eyh = (m3 - xc) * d;
-            // w1*(1/w8), w4*(1/w8): the limiter's normalised face vector
-            // whenever w8 > zerocut; otherwise the edge is cut below
-            const double w33 = exh * xh + eyh * yh;
-            d = -(signF(1.0, w33) * w7);
-            exh = exh * d;
-            eyh = eyh * d;
-            const double w5 = lu;
-            const double w6b = du * exh + dv * eyh;
-            d = DIV(w6b, maxF_nn(w5, zc));
-            edx[is] = edv * du * d;
-            edy[is] = edv * dv * d;
-            if (le_nn(w5, zc) || geF(zc, w6b) || le_nn(w7, zc) || le_nn(w8, zc)) {
-              edx[is] = 0.0;
-              edy[is] = 0.0;
-            }
-          }
-        }
-      }
-      qx[0] = edx[0] - edx[3];
-      qx[1] = edx[1] - edx[0];
-      qx[2] = edx[2] - edx[1];
-      qx[3] = edx[3] - edx[2];
-      qy[0] = edy[0] - edy[3];
-      qy[1] = edy[1] - edy[0];
-      qy[2] = edy[2] - edy[1];
-      qy[3] = edy[3] - edy[2];
-      L::corners(F.cnviscx, iel, qx);
-      L::corners(F.cnviscy, iel, qy);
-      F.visc[iel] = visc;
-    } else {
-      visc = F.visc[iel];
-    }
-    auto corners = [&](double* cx, double* cy) {
+    auto corners = [&](double* x, double* y) {
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        cx[j] = x[j];
-        cy[j] = y[j];
+        x[j] = F.ndx[n[j]];
+        y[j] = F.ndy[n[j]];
       }
     };
-    getdt_tail<L>(F, C, iel, corners, u, v, visc, cflv, cfli, divv, divi);
+    getdt_tail<L>(F, C, iel, corners, u, v, F.visc[iel], cflv, cfli, divv, divi);
   }
   getdt_finish<BS, BATCH>(F, C, S, cflv, cfli, divv, divi, blk0, nblk, el0, I);
 }
-
 #endif
 
 // ================================================================ k_lag_force
@@ -2325,14 +2317,16 @@ int getdt_grid(int nel) { return getdt_blocks(nel, nel); }
 
 // k_edge, k_edgevisc: BS - 2 slots or elements a block
 static_assert(BS_ED == BS_DT, "one edge_grid");
+// the exact build's k_edge: BS / 4 elements a block
+[[maybe_unused]] static int face_grid(int nel) { return (nel + BS_ED / 4 - 1) / (BS_ED / 4); }
 [[maybe_unused]] static int edge_grid(int n) { return (n + BS_ED - 3) / (BS_ED - 2); }
 
 int getdt_launches(const DevCfg& C) {
-#if BL_MIXED
-  return C.ztq ? 1 : 2;
-#else
+#if BL_FAST_ALGEBRA && !BL_MIXED
   (void)C;
-  return BL_FAST_ALGEBRA ? 2 : 1;
+  return 2;
+#else
+  return C.ztq ? 1 : 2;
 #endif
 }
 void launch_getdt(const DevFields& F, const DevCfg& C, cudaStream_t s) {
@@ -2340,6 +2334,8 @@ void launch_getdt(const DevFields& F, const DevCfg& C, cudaStream_t s) {
   if (!C.ztq) k_edgevisc<BS_DT, false><<<edge_grid(F.nel), BS_DT, 0, s>>>(F, C);
 #elif BL_FAST_ALGEBRA
   k_edge<BS_ED, false><<<edge_grid(F.nslot), BS_ED, 0, s>>>(F, C);
+#else
+  if (!C.ztq) k_edge<BS_ED, false><<<face_grid(F.nel), BS_ED, 0, s>>>(F, C);
 #endif
   k_getdt<BS_DT, false><<<getdt_grid(F.nel), BS_DT, 0, s>>>(F, C);
 }
@@ -2380,6 +2376,8 @@ void launch_getdt_batch(const DevFields& F, const DevCfg& C, cudaStream_t s) {
   if (!C.ztq) k_edgevisc<BS_DT, true><<<edge_grid(F.nel), BS_DT, 0, s>>>(F, C);
 #elif BL_FAST_ALGEBRA
   k_edge<BS_ED, true><<<edge_grid(F.nslot), BS_ED, 0, s>>>(F, C);
+#else
+  if (!C.ztq) k_edge<BS_ED, true><<<face_grid(F.nel), BS_ED, 0, s>>>(F, C);
 #endif
   k_getdt<BS_DT, true><<<F.nblk_batch, BS_DT, 0, s>>>(F, C);
 }
