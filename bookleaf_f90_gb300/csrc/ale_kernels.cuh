@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(BS) k_ale_update(DevFields F, DevCfg C) {
     y[j] = F.ndy[n[j]];
   }
   Iso g = getiso(x, y);
-  if (gtF(0.0, g.vol)) atomicMax(&S->negvol_ale, iel + 1 - el_base<BATCH>(F, iel));
+  if (gtF(0.0, g.vol)) note_negvol(F, S, &DevStep::negvol_ale, iel + 1 - el_base<BATCH>(F, iel));
   const double rho = DIV(m1, g.vol);
   double p, cs2;
   eos_pc(C, mat, rho, e, p, cs2);

@@ -200,22 +200,26 @@ int fetch_header(bl_ctx* x, bl_error* e, const char* where) {
   return BL_SUCCESS;
 }
 
-// The per-call entry points queue their kernels and the download of the
-// step header as one replay of a graph captured on first use (again when
-// the kernels' arguments change), then wait for it: one launch instead of
-// one per kernel plus a copy, and the graph's back-to-back kernel launches.
+// The per-call entry points queue their kernels as one replay of a graph
+// captured on first use (again when the kernels' arguments change), then wait
+// for it: one launch instead of one per kernel, and the graph's back-to-back
+// kernel launches.  The kernels keep the header's pinned mirror themselves --
+// the dt reduction's last block writes it, a negative volume raises its field
+// there, for which the header is fetched -- so no copy node ends the graph.
 enum { kCallGetdt = 0, kCallLagstep = 1, kCallAlestep = 2 };
 
 void queue_call_kernels(bl_ctx* x, int which) {
+  bl::DevFields F = x->F;
+  F.hstep = x->hstep;
   if (which == kCallGetdt) {
-    x->L.getdt(x->F, x->C, x->stream);
+    x->L.getdt(F, x->C, x->stream);
   } else if (which == kCallLagstep) {
-    x->L.lag_force(x->F, x->C, x->stream);
-    x->L.lag_accel(x->F, x->C, x->stream);
-    x->L.lag_state(x->F, x->C, x->stream);
-    x->L.mix_closure(x->F, x->C, x->stream);
+    x->L.lag_force(F, x->C, x->stream);
+    x->L.lag_accel(F, x->C, x->stream);
+    x->L.lag_state(F, x->C, x->stream);
+    x->L.mix_closure(F, x->C, x->stream);
   } else {
-    x->L.ale(x->F, x->C, x->stream);
+    x->L.ale(F, x->C, x->stream);
   }
 }
 
@@ -229,7 +233,6 @@ int run_call(bl_ctx* x, int which, bl_error* e, const char* where) {
     r = cudaStreamBeginCapture(x->stream, cudaStreamCaptureModeThreadLocal);
     if (r != cudaSuccess) return cuda_fail(e, r, where);
     queue_call_kernels(x, which);
-    cudaMemcpyAsync(x->hstep, x->F.step, sizeof(DevStep), cudaMemcpyDeviceToHost, x->stream);
     r = cudaStreamEndCapture(x->stream, &g);
     if (r != cudaSuccess) return cuda_fail(e, r, where);
     r = cudaGraphInstantiate(&x->call_exec[which], g, 0);
@@ -247,6 +250,8 @@ int run_call(bl_ctx* x, int which, bl_error* e, const char* where) {
   if (r != cudaSuccess) return cuda_fail(e, r, where);
   r = cudaGetLastError();
   if (r != cudaSuccess) return cuda_fail(e, r, where);
+  if (x->hstep->negvol_pred || x->hstep->negvol_corr || x->hstep->negvol_ale)
+    return fetch_header(x, e, where);
   x->hstep_current = true;
   return BL_SUCCESS;
 }

@@ -129,6 +129,7 @@ struct DevFields {
   double* red_v;             // [2*nblk]
   int* red_i;                // [2*nblk]
   DevStep* step;
+  DevStep* hstep;            // the entry points' calls: the pinned mirror of *step
   StepRec* hist;
   // batch (null in a single-mesh context)
   DevStep* steps;            // [ninst] step headers
@@ -151,6 +152,15 @@ struct DevFields {
 };
 
 // ---------------------------------------------------------------- helpers
+
+// A negative volume of element n (1-based): the largest n in the step header;
+// in a called entry point's mirror any of them, which has the host fetch the
+// header itself.
+__device__ __forceinline__ void note_negvol(const DevFields& F, DevStep* S, int DevStep::*field,
+                                            int n) {
+  atomicMax(&(S->*field), n);
+  if (F.hstep) *const_cast<volatile int*>(&(F.hstep->*field)) = n;
+}
 
 // Fortran MAX/MIN as the CPU restatement evaluates them, (b > a) ? b : a
 // and (b < a) ? b : a: the first argument is returned on ties and when

@@ -654,6 +654,18 @@ __device__ __forceinline__ void block_candidates(double& cflv, int& cfli, double
   warp_div_max(divv, divi);
 }
 
+// The step header as the entry point's host reads it, written by one warp
+// after its lane 0 has finished the header.
+__device__ __forceinline__ void mirror_header(const DevFields& F, const DevStep* S) {
+  __syncwarp();
+  constexpr int N = sizeof(DevStep) / 8;
+  static_assert(sizeof(DevStep) % 8 == 0 && N <= 32, "one word a lane");
+  const int lane = threadIdx.x & 31;
+  if (F.hstep && lane < N)
+    reinterpret_cast<volatile long long*>(F.hstep)[lane] =
+        reinterpret_cast<const volatile long long*>(S)[lane];
+}
+
 // The block reduction of the candidates, the last block's reduction of the
 // block partials and time_dr_end (time_dr_advance.f90:74-132)
 // over the k_getdt blocks [blk0, blk0 + nblk) of one mesh (all of them for
@@ -737,11 +749,13 @@ __device__ __forceinline__ void getdt_finish(const DevFields& F, const DevCfg& C
   if (lane == 0) S->ticket = 0;
   // time_dr_calc candidates then hydro's CFL and DIV (time_dr_advance.f90)
   if (cflv < 0.0) {  // hydro_kn_getdtcfl FAILURE
-    if (lane != 0) return;
-    S->ierr = -1;
-    S->iout = 2;
-    S->err_code = 1;
-    if (run_mode) S->halted = 1;
+    if (lane == 0) {
+      S->ierr = -1;
+      S->iout = 2;
+      S->err_code = 1;
+      if (run_mode) S->halted = 1;
+    }
+    mirror_header(F, S);
     return;
   }
   const double rdt_cfl = s_rdt[0], rdt_div = s_rdt[1];
@@ -760,42 +774,44 @@ __device__ __forceinline__ void getdt_finish(const DevFields& F, const DevCfg& C
   if (gtF(mind, rdt_cfl)) { mind = rdt_cfl; mins = 3; }
   if (gtF(mind, rdt_div)) { mind = rdt_div; mins = 4; }
   const double rdt = __shfl_sync(0xffffffffu, inv, mins);
-  if (lane != 0) return;
-  // 1-based element numbers local to the mesh (0: none)
-  const int cfln = cfli >= 0 && cfli != 0x7fffffff ? cfli - el0 + 1 : 0;
-  const int divn = divi >= 0 ? divi - el0 + 1 : 0;
-  const int mini = mins == 3 ? cfln : (mins == 4 ? divn : -1);
-  const double time = time0 + mind;
-  S->cfl_rdt = rdt_cfl;
-  S->cfl_idt = cfln;
-  S->div_rdt = rdt_div;
-  S->div_idt = divn;
-  S->nstep = nstep0 + 1;
-  S->dt = mind;
-  S->rdt = rdt;
-  S->sdt = mins;
-  S->idtel = mini;
-  S->time = time;
-  const bool low = gtF(dt_min, mind);
-  if (low) {
-    S->ierr = -1;
-    S->iout = 1;
-    S->err_code = 2;
-    if (run_mode) S->halted = 1;
-  }
-  if (run_mode) {
-    if (geF(time, time_end)) S->stop_next = 1;
-    if (F.hist && nrec0 < C.max_records) {
-      StepRec& r = F.hist[nrec0];
-      r.time = time;
-      r.dt = mind;
-      r.nstep = nstep0 + 1;
-      r.idtel = mini;
-      r.sdt_code = mins;
-      r.ierr = low ? -1 : S->ierr;
+  if (lane == 0) {
+    // 1-based element numbers local to the mesh (0: none)
+    const int cfln = cfli >= 0 && cfli != 0x7fffffff ? cfli - el0 + 1 : 0;
+    const int divn = divi >= 0 ? divi - el0 + 1 : 0;
+    const int mini = mins == 3 ? cfln : (mins == 4 ? divn : -1);
+    const double time = time0 + mind;
+    S->cfl_rdt = rdt_cfl;
+    S->cfl_idt = cfln;
+    S->div_rdt = rdt_div;
+    S->div_idt = divn;
+    S->nstep = nstep0 + 1;
+    S->dt = mind;
+    S->rdt = rdt;
+    S->sdt = mins;
+    S->idtel = mini;
+    S->time = time;
+    const bool low = gtF(dt_min, mind);
+    if (low) {
+      S->ierr = -1;
+      S->iout = 1;
+      S->err_code = 2;
+      if (run_mode) S->halted = 1;
     }
-    S->nrecord = nrec0 + 1;
+    if (run_mode) {
+      if (geF(time, time_end)) S->stop_next = 1;
+      if (F.hist && nrec0 < C.max_records) {
+        StepRec& r = F.hist[nrec0];
+        r.time = time;
+        r.dt = mind;
+        r.nstep = nstep0 + 1;
+        r.idtel = mini;
+        r.sdt_code = mins;
+        r.ierr = low ? -1 : S->ierr;
+      }
+      S->nrecord = nrec0 + 1;
+    }
   }
+  mirror_header(F, S);
 }
 
 // Consecutive tiles of BS elements that a k_getdt block of the fast and mixed
@@ -1780,7 +1796,7 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
     }
     g = getiso(xh, yh);
   }
-  if (gtF(0.0, g.vol)) atomicMax(&S->negvol_pred, iel + 1 - el_base<BATCH>(F, iel));
+  if (gtF(0.0, g.vol)) note_negvol(F, S, &DevStep::negvol_pred, iel + 1 - el_base<BATCH>(F, iel));
   const double rho = DIV(m, g.vol);
   // ---- energy (hydro_kn_getenergy with dts = dt/2) and EoS
   const double eh = e0 - DIV(work, maxF(m, zc)) * hdt;
@@ -1916,7 +1932,7 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
   }
   // ---- geometry, density (geometry_dr_getgeometry, density_dr_getdensity)
   Iso g = getiso(xh, yh);
-  if (gtF(0.0, g.vol)) atomicMax(&S->negvol_pred, iel + 1 - el_base<BATCH>(F, iel));
+  if (gtF(0.0, g.vol)) note_negvol(F, S, &DevStep::negvol_pred, iel + 1 - el_base<BATCH>(F, iel));
   const double rho = DIV(m, g.vol);
   // ---- energy (hydro_kn_getenergy with dts = dt/2) and EoS
   const double eh = energy_update(e0, m, zc, hdt, fx, fy, u, v);
@@ -2101,7 +2117,7 @@ __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
   const EosTab mat = eos_tab(C, __ldg(F.ielmat + iel));
   const double m = F.mass[iel], e0 = F.e[iel];
   Iso g = getiso(x, y);
-  if (gtF(0.0, g.vol)) atomicMax(&S->negvol_corr, iel + 1 - el_base<BATCH>(F, iel));
+  if (gtF(0.0, g.vol)) note_negvol(F, S, &DevStep::negvol_corr, iel + 1 - el_base<BATCH>(F, iel));
   const double rho = DIV(m, g.vol);
   const d4 f4x = F.cnfx[iel], f4y = F.cnfy[iel];
   const double fx[4] = {f4x.x, f4x.y, f4x.z, f4x.w};
