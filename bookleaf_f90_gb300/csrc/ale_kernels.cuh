@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(BS) k_ale_update(DevFields F, DevCfg C) {
 }
 
 static constexpr int BS_A = 128;
-static constexpr int BS_AN = 256;
+static constexpr int BS_AN = 64;
 
 template <bool BATCH>
 void launch_ale_t(const DevFields& F, const DevCfg& C, cudaStream_t s) {

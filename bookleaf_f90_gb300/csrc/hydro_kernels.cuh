@@ -62,14 +62,15 @@ static __device__ __noinline__ double dsqrt_call(double x) { return dsqrt_rn(x);
 #define SQRT(a) ::bl::dsqrt_rn(a)
 #endif
 
-// Resident blocks of 128 threads per SM the two heaviest kernels are
-// compiled for (register budget 65536 / (128 * n) per thread).  Chosen by
-// timing the whole Sedov 512x512 run on the GB300 over k_getdt n = 5..8
-// and k_lag_force n = 2..6: 832.0M zone-cycles/s at 7 and 4 against 814.9M
-// at 5 and 3, 822.0M at 7 and 3, 823.4M at 5 and 4.  k_getdt gains from
-// the warps that hide its integer-pipe divide chains and from the 8,192
-// warps of a 512x512 mesh filling 1.92 waves of 28 warps per SM instead of
-// 2.69 waves of 20 (the last, part-filled wave drains at low occupancy).
+// Resident blocks per SM that the edge and candidate kernels (of 128 threads)
+// and k_lag_force (of 64) are compiled for.  All are bound by the FP64 pipe,
+// which two or three warps a scheduler fill as long as their integer divide
+// chains overlap, so the bound is the register count that spills nothing.
+// k_getdt at 4/5/6/7/8 blocks: Sedov 512x512 (with the edge kernel)
+// 75/73/72/69/69 us.  k_lag_force at 3/4/5/6 blocks of 128: 100/90/90/91 us
+// with sub-zonal and hourglass forces; five is faster by 8 % where the mesh
+// fits one wave of five and not of four (280x280 to 301x301) and slower by 6
+// to 9 % at 200x200, 330x330 and 450x450.
 #ifndef BL_GETDT_MINB
 #define BL_GETDT_MINB 7
 #endif
@@ -80,7 +81,7 @@ static __device__ __noinline__ double dsqrt_call(double x) { return dsqrt_rn(x);
 #define BL_FAST_ALGEBRA 0
 #endif
 #ifndef BL_FORCE_MINB
-#define BL_FORCE_MINB 4
+#define BL_FORCE_MINB 8
 #endif
 // Minimum resident blocks per SM of the two short kernels (0: the plain
 // block-size bound).  From the same whole-run sweep: k_lag_accel with a
@@ -2318,7 +2319,7 @@ __global__ void __launch_bounds__(32 * kClosureWarps) k_mix_closure(DevFields F,
 // ================================================================ launchers
 
 static constexpr int BS_DT = 128;
-static constexpr int BS_EL = 128;
+static constexpr int BS_EL = 64;   // k_lag_force, k_lag_state
 static constexpr int BS_ED = 128;  // k_edge
 static constexpr int BS_ND = 128;
 
