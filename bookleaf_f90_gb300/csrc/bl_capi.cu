@@ -200,6 +200,24 @@ int fetch_header(bl_ctx* x, bl_error* e, const char* where) {
   return BL_SUCCESS;
 }
 
+// k_lag_state and, with the learned closure on, k_mix_closure beside it: the
+// closure's blocks come first, so that they start first.  What the context's
+// stream gets next waits for both.  A step of the device loop with one after
+// the other and with both at once: two materials on 100x10 cells 48.3 and 44.0
+// us, on 800x80 71.7 and 67.4 us, on 1600x160 164.7 and 149.0 us.
+template <class State, class Mix>
+void queue_state(bl_ctx* x, State state, Mix mix, const bl::DevFields& F, const bl::DevCfg& C) {
+  const bool learned = F.closure && F.nmx > 0;
+  if (learned) {
+    cudaEventRecord(x->fork, x->stream);
+    cudaStreamWaitEvent(x->side, x->fork, 0);
+    mix(F, C, x->side);
+    cudaEventRecord(x->join, x->side);
+  }
+  state(F, C, x->stream);
+  if (learned) cudaStreamWaitEvent(x->stream, x->join, 0);
+}
+
 // The per-call entry points queue their kernels as one replay of a graph
 // captured on first use (again when the kernels' arguments change), then wait
 // for it: one launch instead of one per kernel, and the graph's back-to-back
@@ -216,8 +234,7 @@ void queue_call_kernels(bl_ctx* x, int which) {
   } else if (which == kCallLagstep) {
     x->L.lag_force(F, x->C, x->stream);
     x->L.lag_accel(F, x->C, x->stream);
-    x->L.lag_state(F, x->C, x->stream);
-    x->L.mix_closure(F, x->C, x->stream);
+    queue_state(x, x->L.lag_state, x->L.mix_closure, F, x->C);
   } else {
     x->L.ale(F, x->C, x->stream);
   }
@@ -743,6 +760,9 @@ int bl_finalize(bl_ctx* x) {
   if (x->F.hist) cudaFree(x->F.hist);
   if (x->diag) cudaFree(x->diag);
   if (x->hstep) cudaFreeHost(x->hstep);
+  if (x->fork) cudaEventDestroy(x->fork);
+  if (x->join) cudaEventDestroy(x->join);
+  if (x->side) cudaStreamDestroy(x->side);
   if (x->stream) cudaStreamDestroy(x->stream);
   delete x;
   return BL_SUCCESS;
@@ -858,8 +878,7 @@ int bl_run(bl_ctx* x, bl_timestep* ts, int max_steps, bl_step_record* history, i
       x->L.getdt(F, C, x->stream);
       x->L.lag_force(F, C, x->stream);
       x->L.lag_accel(F, C, x->stream);
-      x->L.lag_state(F, C, x->stream);
-      x->L.mix_closure(F, C, x->stream);
+      queue_state(x, x->L.lag_state, x->L.mix_closure, F, C);
       if (with_ale) x->L.ale(F, C, x->stream);
     }
     r = cudaStreamEndCapture(x->stream, &g);
@@ -890,8 +909,7 @@ int bl_run(bl_ctx* x, bl_timestep* ts, int max_steps, bl_step_record* history, i
         x->L.getdt(F, C, x->stream);
         x->L.lag_force(F, C, x->stream);
         x->L.lag_accel(F, C, x->stream);
-        x->L.lag_state(F, C, x->stream);
-        x->L.mix_closure(F, C, x->stream);
+        queue_state(x, x->L.lag_state, x->L.mix_closure, F, C);
         if (with_ale) x->L.ale(F, C, x->stream);
       }
       x->launches += (long long)remaining * per_step;
@@ -974,8 +992,7 @@ int bl_time_step_kernels(bl_ctx* x, bl_timestep* ts, int nstep, double* ms, int 
     cudaEventRecord(ev[4 * k + 2], x->stream);
     x->L.lag_accel(x->F, x->C, x->stream);
     cudaEventRecord(ev[4 * k + 3], x->stream);
-    x->L.lag_state(x->F, x->C, x->stream);
-    x->L.mix_closure(x->F, x->C, x->stream);
+    queue_state(x, x->L.lag_state, x->L.mix_closure, x->F, x->C);
     cudaEventRecord(ev[4 * k + 4], x->stream);
   }
   x->launches += (long long)nstep * (x->L.getdt_launches(x->C) + bl::launches_lagstep(x->F));
@@ -1703,8 +1720,7 @@ int bl_run_batch(bl_ctx* x, bl_timestep* ts, int max_steps, int* status, int* ns
     x->L.getdt_b(F, C, x->stream);
     x->L.lag_force_b(F, C, x->stream);
     x->L.lag_accel_b(F, C, x->stream);
-    x->L.lag_state_b(F, C, x->stream);
-    x->L.mix_closure_b(F, C, x->stream);
+    queue_state(x, x->L.lag_state_b, x->L.mix_closure_b, F, C);
     if (with_ale) x->L.ale_b(F, C, x->stream);
   };
   if (!x->bexec || x->b_ale != with_ale || x->b_gsteps != G || x->b_ndblock != F.nd_block) {
@@ -1792,6 +1808,10 @@ int bl_set_closure(bl_ctx* x, bl_mlp* net, const float* norm, int on, bl_error* 
   bl::DevFields& F = x->F;
   if (on) {
     cudaError_t st = cudaSuccess;
+    if (!x->side) st = cudaStreamCreateWithFlags(&x->side, cudaStreamNonBlocking);
+    if (st == cudaSuccess && !x->fork) st = cudaEventCreateWithFlags(&x->fork, cudaEventDisableTiming);
+    if (st == cudaSuccess && !x->join) st = cudaEventCreateWithFlags(&x->join, cudaEventDisableTiming);
+    if (st != cudaSuccess) return cuda_fail(e, st, "bl_set_closure");
     if (!F.mxv0) F.mxv0 = dalloc<double>(x, std::max(1, x->s.nmx), st);
     if (!F.mlp_norm) F.mlp_norm = dalloc<float>(x, 2 * BL_MLP_IN + 2, st);
     if (!F.mlp_count) F.mlp_count = dalloc<unsigned long long>(x, 2, st);

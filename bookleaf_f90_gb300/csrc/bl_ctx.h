@@ -31,9 +31,12 @@ struct bl_ctx {
   bool hstep_current = false;
   bool cs2_is_v = false;     // elcs2 currently holds cs2 + elvisc (after getdt)
   long long launches = 0;
+  // the learned closure's branch beside k_lag_state (queue_state), forked from
+  // and joined to `stream`
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   // per-call entry points: one cached graph each (getdt, lagstep, alestep)
-  // of their kernels and the header download, with the kernel arguments it
-  // was captured with
+  // of their kernels, with the kernel arguments it was captured with
   cudaGraphExec_t call_exec[3] = {nullptr, nullptr, nullptr};
   bl::DevFields call_F[3] = {};
   bl::DevCfg call_C[3] = {};

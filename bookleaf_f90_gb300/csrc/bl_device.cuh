@@ -147,7 +147,7 @@ struct DevFields {
                              // image (bl_mma.cuh), copied at bl_set_closure
   const float* mlp_norm;     // [22]: feature means, inverse spreads, output
                              // scale, conservation tolerance
-  double* mxv0;              // [nmx] cell volume at the start of the step
+  double* mxv0;              // [nmx] cell volume at the start of the step (k_lag_force)
   unsigned long long* mlp_count;  // [2]: cells the closure saw, cells it rejected
 };
 

@@ -1807,6 +1807,7 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
   // ---- mixed cells: component state at the half step
   if (imx >= 0) {
     const int c0 = F.imxfcp[imx], nc = F.imxncp[imx];
+    if (F.closure && nc == 2) F.mxv0[imx] = F.vol[iel];  // for k_mix_closure
     double ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
     for (int k = 0; k < nc; k++) {
       const int icp = c0 + k;
@@ -1942,6 +1943,7 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
   // ---- mixed cells: component state at the half step
   if (imx >= 0) {
     const int c0 = F.imxfcp[imx], nc = F.imxncp[imx];
+    if (F.closure && nc == 2) F.mxv0[imx] = F.vol[iel];  // for k_mix_closure
     double ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
     for (int k = 0; k < nc; k++) {
       const int icp = c0 + k;
@@ -2143,11 +2145,9 @@ __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
   }
   F.cnwt[iel] = make_d4(g.w0, g.w1, g.w2, g.w3);
   const int imx = F.elmx ? F.elmx[iel] : -1;
-  // the learned closure (k_mix_closure, launched next) splits a two-material
-  // cell's volume change between its materials and updates them: it needs
-  // the cell volume at the start of the step
+  // the learned closure (k_mix_closure, beside this kernel) splits a
+  // two-material cell's volume change between its materials and updates them
   const bool learned = imx >= 0 && F.closure && F.imxncp[imx] == 2;
-  if (learned) F.mxv0[imx] = F.vol[iel];
   F.vol[iel] = g.vol;
   F.rho[iel] = rho;
   F.e[iel] = e;
@@ -2181,7 +2181,7 @@ __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
 
 // ================================================================ k_mix_closure
 
-// The learned mixed-cell closure, after k_lag_state.  For each two-material
+// The learned mixed-cell closure, beside k_lag_state.  For each two-material
 // cell the network (tensor cores, 16 cells per warp) predicts the volume
 // each material gains over the step beyond the plain closure's share (its
 // volume fraction of the cell's change), as a fraction of the cell's volume
@@ -2208,6 +2208,13 @@ __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
 // volume and total energy, and every element and node field of the step,
 // are the plain closure's, and a rejected cell ends exactly as under it.
 // In a batch each cell reads the step header of its own mesh.
+//
+// One dependent chain of loads, network, divides and FP64 on a few warps: 12
+// us whatever the number of cells, up to a few thousand.  So it runs beside
+// k_lag_state, on a branch of its own (queue_state): the cell's volume at the
+// start of the step comes from k_lag_force, the one at its end from the
+// vertices, and nothing that one of the two kernels writes is read by the
+// other.
 constexpr int kClosureWarps = 4;
 template <bool BATCH>
 __global__ void __launch_bounds__(32 * kClosureWarps) k_mix_closure(DevFields F, DevCfg C) {
@@ -2226,6 +2233,8 @@ __global__ void __launch_bounds__(32 * kClosureWarps) k_mix_closure(DevFields F,
   const bool two = imx < F.nmx && F.imxncp[imx] == 2;
   const int iel = two ? F.imxel[imx] : 0;
   const DevStep* S = el_step<BATCH>(F, iel);
+  const int4 nd = __ldg(F.ielnd + iel);
+  const int n[4] = {nd.x, nd.y, nd.z, nd.w};
   const bool cell = two && !halted(S);
   const double dt = cell ? S->dt : 0.0;
   double V0 = 0.0, V1 = 0.0;
@@ -2233,7 +2242,13 @@ __global__ void __launch_bounds__(32 * kClosureWarps) k_mix_closure(DevFields F,
   if (cell) {
     c0 = F.imxfcp[imx];
     V0 = F.mxv0[imx];
-    V1 = F.vol[iel];
+    double x[4], y[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      x[j] = F.ndx[n[j]];
+      y[j] = F.ndy[n[j]];
+    }
+    V1 = getiso(x, y).vol;
   }
   if (lane < 16) {
     float f[mlp::NI];
@@ -2263,8 +2278,6 @@ __global__ void __launch_bounds__(32 * kClosureWarps) k_mix_closure(DevFields F,
     fr[1] = F.frvol[c0 + 1];
     pbar = fr[0] * F.cpp[c0] + fr[1] * F.cpp[c0 + 1];
     const double frk = k ? fr[1] : fr[0];
-    const int4 nd = __ldg(F.ielnd + iel);
-    const int n[4] = {nd.x, nd.y, nd.z, nd.w};
     const d4 a = F.cpfx[icp], b = F.cpfy[icp];
     const double cfx[4] = {a.x, a.y, a.z, a.w}, cfy[4] = {b.x, b.y, b.z, b.w};
     double cu[4], cv[4];
