@@ -34,6 +34,13 @@
 #include "bl_kernels.h"
 #include "bl_mma.cuh"
 
+// The fast build may also use exact algebraic identities that can change
+// only the sign of a zero (negation symmetry of opposite corners); the
+// exact build evaluates every expression as written.
+#ifndef BL_FAST_ALGEBRA
+#define BL_FAST_ALGEBRA 0
+#endif
+
 // Every FP64 division and square root of the per-element work goes
 // through the integer-pipe versions, which return the IEEE results bit for
 // bit (bl_fp64.cuh); the three of the dt reduction's last block, one
@@ -61,6 +68,17 @@ static __device__ __noinline__ double dsqrt_call(double x) { return dsqrt_rn(x);
 #ifndef SQRT
 #define SQRT(a) ::bl::dsqrt_rn(a)
 #endif
+// Inlined divides, for k_lag_force and k_lag_accel of the fast and mixed
+// builds: few enough to fit, and the independent ones (four sub-zonal
+// densities; two components of an acceleration) overlap.  Called and inlined,
+// a step of Sedov 301x301 in the mixed build 80.0 and 78.9 us, of 512x512 185.0
+// and 183.7 (fast), 175.1 and 173.9 us (mixed), of the 300x120 polar Noh 40.0
+// and 39.4 us.
+#if BL_FAST_ALGEBRA
+#define DIV_IN(a, b) ::bl::ddiv_rn((a), (b))
+#else
+#define DIV_IN(a, b) DIV(a, b)
+#endif
 
 // Resident blocks per SM that the edge and candidate kernels (of 128 threads)
 // and k_lag_force (of 64) are compiled for.  All are bound by the FP64 pipe,
@@ -73,12 +91,6 @@ static __device__ __noinline__ double dsqrt_call(double x) { return dsqrt_rn(x);
 // to 9 % at 200x200, 330x330 and 450x450.
 #ifndef BL_GETDT_MINB
 #define BL_GETDT_MINB 7
-#endif
-// The fast build may also use exact algebraic identities that can change
-// only the sign of a zero (negation symmetry of opposite corners); the
-// exact build evaluates every expression as written.
-#ifndef BL_FAST_ALGEBRA
-#define BL_FAST_ALGEBRA 0
 #endif
 #ifndef BL_FORCE_MINB
 #define BL_FORCE_MINB 8
@@ -1701,10 +1713,10 @@ struct SubZone {
 };
 __device__ __forceinline__ SubZone sub_zone(double cross, double ts, double td, const d4& spm) {
   SubZone z;
-  z.q[0] = DIV(spm.x, fma(td, 0.5, cross));
-  z.q[1] = DIV(spm.y, fma(ts, 0.5, cross));
-  z.q[2] = DIV(spm.z, fma(-td, 0.5, cross));
-  z.q[3] = DIV(spm.w, fma(-ts, 0.5, cross));
+  z.q[0] = DIV_IN(spm.x, fma(td, 0.5, cross));
+  z.q[1] = DIV_IN(spm.y, fma(ts, 0.5, cross));
+  z.q[2] = DIV_IN(spm.z, fma(-td, 0.5, cross));
+  z.q[3] = DIV_IN(spm.w, fma(-ts, 0.5, cross));
   return z;
 }
 // one direction's corner forces (sg = 1: x from the b's, -1: y from the
@@ -1798,9 +1810,9 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
     g = getiso(xh, yh);
   }
   if (gtF(0.0, g.vol)) note_negvol(F, S, &DevStep::negvol_pred, iel + 1 - el_base<BATCH>(F, iel));
-  const double rho = DIV(m, g.vol);
+  const double rho = DIV_IN(m, g.vol);
   // ---- energy (hydro_kn_getenergy with dts = dt/2) and EoS
-  const double eh = e0 - DIV(work, maxF(m, zc)) * hdt;
+  const double eh = e0 - DIV_IN(work, maxF(m, zc)) * hdt;
   double ph, cs2h;
   eos_pc(C, mat, rho, eh, ph, cs2h);
   double fx[4], fy[4];
@@ -2035,8 +2047,8 @@ __global__ void BL_ACCEL_BOUNDS(BS) k_lag_accel(DevFields F, DevCfg C) {
   const double w1 = C.dencut * nda;
   double ax, ay;
   if (gtF(ndm, w1)) {
-    ax = DIV(fx, ndm);
-    ay = DIV(fy, ndm);
+    ax = DIV_IN(fx, ndm);
+    ay = DIV_IN(fy, ndm);
   } else {
     ax = 0.0;
     ay = 0.0;
