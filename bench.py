@@ -17,7 +17,7 @@ e2e        the same metric through the reference-facing C-ABI with host
            buffers: bl_init (upload of every registered host field), K calls
            each of bl_getdt/bl_lagstep(/bl_alestep) and bl_sync_to_host of
            the whole state, all inside the timed region.
-roofline   the dominant kernel (edge viscosity + dt, k_getdt) against the
+roofline   the longest kernel of the step against the
            measured HBM copy bandwidth, with algorithmic bytes per zone
            (each field read once plus each field written once); "fp64"
            reports the binding FP64 issue roof.
@@ -46,16 +46,17 @@ sys.path.insert(0, HERE)
 # per node)
 B_LAG = 724
 B_EUL = 1628
-B_GETDT = 164
+# the same for each entry of kernels_ms (k_getdt: with the edge kernel before it)
+B_KERNEL = {"k_getdt": 164, "k_lag_force": 192, "k_lag_accel": 200, "k_lag_state": 168}
 # the headline metric, printed by both arms
 METRIC = "zone-cycles/s FP64 (1 GB300, %HBM roof); batched+MLP vs plain GPU at stated L1 err"
 
 
-def load_profile(name="k_getdt_current.json"):
-    """The committed summary of the latest single-kernel ncu capture of
-    k_getdt (profiles/k_getdt_current.json): its FP64-pipe thread
-    instructions per zone and DRAM bytes per launch, with the command and
-    mesh size they were taken at; None where absent."""
+def load_profile(name="lagrangian_kernels_current.json"):
+    """The committed summary of the latest ncu capture of the Lagrangian
+    step's kernels (profiles/lagrangian_kernels_current.json): their FP64-pipe
+    thread instructions per zone and DRAM bytes per launch, with the command
+    and mesh size they were taken at; None where absent."""
     path = os.path.join(HERE, "profiles", name)
     if not os.path.exists(path):
         return None
@@ -990,50 +991,55 @@ def main():
     p.timestep = ts
 
     # ---------------- per-kernel durations at the end-of-run state --------
-    # 16 more steps at the state the run left, the four kernels of each
-    # queued back to back on the library's stream with CUDA events between
-    # them (no host copies): the mean duration of each kernel.  The profiler
-    # range brackets these launches only, so that an ncu capture with
-    # --profile-from-start off sees the same launches.
+    # 16 more steps at the state the run left, the kernels of each queued
+    # back to back on the library's stream with CUDA events between them (no
+    # host copies): the mean duration of each.  The profiler range brackets
+    # these launches only, so that an ncu capture with --profile-from-start
+    # off sees the same launches.
     torch.cuda.profiler.start()
     ierr_k, kms = s.time_step_kernels(16, p.timestep.copy())
     torch.cuda.profiler.stop()
     assert ierr_k == 0, s.error.message
-    k_ms = kms[0]
+    kernels_ms = dict(zip(B_KERNEL, kms))
+    longest = max(kernels_ms, key=kernels_ms.get)
+    k_ms = kernels_ms[longest]
     lag_ms = kms[1] + kms[2] + kms[3]
     hbm_peak, peak_kind = load_peaks()
-    achieved = B_GETDT * nel / (k_ms * 1e-3) / 1e9
+    achieved = B_KERNEL[longest] * nel / (k_ms * 1e-3) / 1e9
     prof = load_profile()
     # the capture's figures hold for the FP64 (fast) build on the default
     # workload, where they were taken; elsewhere the line reports none
     if prof and (args.fp != "fast" or not wname.startswith("sedov_512x512_lagrangian")):
         prof = None
-    traffic = (prof["dram_bytes_per_launch"] * nel / prof["nel"]) if prof else None
+    # k_getdt's duration is that of the edge kernel and its own
+    of = [prof["kernels"][k] for k in
+          (("k_edge", "k_getdt") if longest == "k_getdt" else (longest,))] if prof else []
+    traffic = sum(k["dram_bytes_per_launch"] for k in of) * nel / prof["nel"] if prof else None
     roof = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
             "frac": achieved / hbm_peak, "traffic": traffic,
-            "traffic_unit": "bytes per launch, from profiles/k_getdt_current.json (ncu, "
+            "traffic_unit": "bytes per launch, from profiles/lagrangian_kernels_current.json (ncu, "
                             "dram__bytes_read.sum + dram__bytes_write.sum%s)"
                             % ("" if not prof or prof["nel"] == nel else
                                ", scaled from %d zones" % prof["nel"]),
-            "kernel": "k_getdt",
+            "kernel": longest,
             "peak_kind": peak_kind, "kernel_ms": k_ms,
             "note": "the FP64 issue rate, not HBM, bounds this path; see fp64",
             "lagstep_ms": lag_ms,
-            "kernels_ms": {"k_getdt": kms[0], "k_lag_force": kms[1], "k_lag_accel": kms[2],
-                           "k_lag_state": kms[3],
-                           "how": "mean of 16 steps after the timed run, CUDA events between "
-                                  "the kernels on the library's stream"}}
+            "kernels_ms": dict(kernels_ms,
+                               how="mean of 16 steps after the timed run, CUDA events between "
+                                   "the kernels on the library's stream; k_getdt: the edge "
+                                   "kernel and k_getdt")}
     step_bytes = bytes_zc * nel
     from bookleaf_f90_gb300 import _lib
     rates = _lib.fp64_rates()
-    ipz = prof["fp64_pipe_instr_per_zone"] if prof else None
+    ipz = sum(k["fp64_pipe_instr_per_zone"] for k in of) if prof else None
     fp64_ach = ipz * nel / (k_ms * 1e-3) / 1e9 if ipz else None
-    fp64 = {"bound": "fp64", "kernel": "k_getdt", "unit": "G FP64-pipe instr/s",
+    fp64 = {"bound": "fp64", "kernel": longest, "unit": "G FP64-pipe instr/s",
             "achieved": fp64_ach, "peak": rates["dfma"],
             "frac": fp64_ach / rates["dfma"] if ipz else None,
             "peak_kind": "measured live (DFMA issue loop, bl_fp64_rates)",
             "instr_per_zone": ipz,
-            "instr_source": "profiles/k_getdt_current.json: %s" % (
+            "instr_source": "profiles/lagrangian_kernels_current.json: %s" % (
                 prof["how"] if prof else
                 "not applicable: the capture is of the FP64 (fast) build on Sedov 512x512"),
             "rates_gops": rates,

@@ -1,12 +1,16 @@
 // hydro_kernels.cu -- the Lagrangian hot path on sm_103a.
 //
-// Four kernels per step replace the reference's sequence of loops:
-//   k_getdt        inf_solver_getdt: utils_kn_cngather u,v; the three edge-
-//                  viscosity loops (hydro_kn_edgeviscosity.f90:30-282);
-//                  hydro_dr_getcs2; hydro_kn_getdtcfl / getdtdiv
-//                  (hydro_kn_getdt.f90:30-122) with the two argmin/argmax
-//                  scans done as a block reduction plus a last-block pass
-//                  that also runs time_dr_end (time_dr_advance.f90:74-132).
+// Five kernels per step replace the reference's sequence of loops:
+//   k_edge         the three edge-viscosity loops of inf_solver_getdt
+//                  (hydro_kn_edgeviscosity.f90:30-282), with utils_kn_cngather
+//                  of u,v: each edge of the mesh once (fast build), each face
+//                  of each element (exact build), each element (mixed build,
+//                  where it is k_edgevisc).
+//   k_getdt        the corner viscosities; hydro_dr_getcs2; hydro_kn_getdtcfl /
+//                  getdtdiv (hydro_kn_getdt.f90:30-122) with the two
+//                  argmin/argmax scans done as a block reduction plus a
+//                  last-block pass that also runs time_dr_end
+//                  (time_dr_advance.f90:74-132).
 //   k_lag_force    inf_solver_lagstep up to the corrector force: predictor
 //                  force (hydro_kn_getforce.f90), half-step vertices,
 //                  geometry, density, energy, EoS, then the corrector force
@@ -19,10 +23,12 @@
 //   k_lag_state    the corrector getstate: geometry at x^{n+1}, density,
 //                  energy from e^n with the corrector forces and ubar, EoS.
 //
-// Every expression keeps the reference's operand order.  This file is
-// compiled twice: with --fmad=false (namespace exact) the results equal the
-// CPU restatement bit for bit; with --fmad=true (namespace fast) the compiler
-// may fuse multiply-adds.
+// This file is compiled three times.  With --fmad=false (namespace exact) every
+// expression keeps the reference's operand order and the results equal the CPU
+// restatement bit for bit; with --fmad=true (namespace fast) the compiler may
+// fuse multiply-adds and algebraic identities are used (BL_FAST_ALGEBRA);
+// namespace mixed is the fast build with the edge viscosity and the limiters
+// in FP32 (BL_MIXED).
 #pragma once
 #include <cfloat>
 #include <cmath>
@@ -48,9 +54,10 @@
 // a fraction of the latency).
 // The divides and square roots run out of line: one body per kernel instead
 // of ~60 inlined copies of ~100 instructions, which overflowed the
-// instruction cache (k_getdt stalled on instruction fetch); measured on the
-// GB300 over the whole Sedov 512x512 run: 556.1M zone-cycles/s against
-// 514.6M inlined.
+// instruction cache (the getdt kernels stalled on instruction fetch).
+// Inlined throughout this file, a step of Sedov 512x512 takes 185.8 us against 185.8
+// (fast) and 588 against 581 us (exact), k_lag_state of Noh 1024x1024 Eulerian
+// 84 against 82 us; two kernels gain (DIV_IN below).
 #ifndef BL_DIV_CALL
 #define BL_DIV_CALL 1
 #endif
@@ -96,11 +103,10 @@ static __device__ __noinline__ double dsqrt_call(double x) { return dsqrt_rn(x);
 #define BL_FORCE_MINB 8
 #endif
 // Minimum resident blocks per SM of the two short kernels (0: the plain
-// block-size bound).  From the same whole-run sweep: k_lag_accel with a
-// one-block bound takes 56 registers and no spills (24.8 us against 26.3 us
-// at the 40 registers of the plain bound, 913.7M against 907.8M
-// zone-cycles/s); k_lag_state is best with the plain bound (72 registers;
-// 1, 8, 12 and 16 blocks were slower or equal).
+// block-size bound), from sweeps of Sedov 512x512: k_lag_accel with a
+// one-block bound keeps its gathers in registers (24.8 us against 26.3 us at
+// the 40 registers of the plain bound); k_lag_state is best with the plain
+// bound (80 registers; 1, 8, 12 and 16 blocks were slower or equal).
 #ifndef BL_ACCEL_MINB
 #define BL_ACCEL_MINB 1
 #endif

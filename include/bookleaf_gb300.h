@@ -317,7 +317,8 @@ long long bl_kernel_launches(bl_ctx *ctx);
  * with a CUDA event between each and no host copy between steps, without
  * the end-time stop of bl_run (so it also runs past time_end).  ms[0..3]
  * (n >= 4) receive the mean durations in milliseconds of the getdt
- * kernel and of the three lagstep kernels (force, acceleration, state);
+ * kernels and of the three lagstep kernels (force, acceleration, state --
+ * with the learned closure's beside it);
  * *ts receives the state after the last step.  The ALE step is not run.
  * Returns BL_SUCCESS, or BL_FAILURE with *err set as the solver entry
  * points set it. */
@@ -397,7 +398,7 @@ typedef struct {
  * allocating behind its back would fail or break its accounting.  It runs
  * bl_getdt's computation (edge viscosity, elcs2+elvisc, CFL and divergence
  * limits, time_dr_calc/time_dr_end) on arrays the caller passes, without a
- * bl_ctx: the library's own exact-form getdt kernel, so its results equal
+ * bl_ctx: the library's own exact-form getdt kernels, so its results equal
  * bl_getdt's in BL_FP_EXACT mode bit for bit.  Its reduction scratch is a fixed file-scope device
  * array, held by every GPU that loads the library until the process exits;
  * nothing is allocated or freed by this call.  The first call on a device
