@@ -99,8 +99,14 @@ static __device__ __noinline__ double dsqrt_call(double x) { return dsqrt_rn(x);
 #ifndef BL_GETDT_MINB
 #define BL_GETDT_MINB 7
 #endif
+// The exact build's k_lag_force spills at any of these and gains from warps:
+// 8/9/10/12 blocks 268/261/256/258 us on Sedov 512x512, 55/53/52/53 on 200x200.
 #ifndef BL_FORCE_MINB
+#if BL_FAST_ALGEBRA
 #define BL_FORCE_MINB 8
+#else
+#define BL_FORCE_MINB 10
+#endif
 #endif
 // Minimum resident blocks per SM of the two short kernels (0: the plain
 // block-size bound), from sweeps of Sedov 512x512: k_lag_accel with a
@@ -350,6 +356,19 @@ __device__ __forceinline__ double min_dlm(const double* x, const double* y) {
   return m;
 }
 
+#if !BL_FAST_ALGEBRA
+// Rounding is symmetric: -a + b is a - b with the other sign, and so is a
+// product with it, bit for bit -- except that a zero's sign is the
+// expression's own (a - b and -a + b are both +0 where a = b).  The exact
+// build negates on the integer pipe and evaluates the expression only where
+// one of the sums is zero: 80 of the 480 FP64 instructions of k_lag_force
+// fewer, Sedov 512x512 292 -> 268 us.
+__device__ __forceinline__ bool any_zero(double a, double b, double c, double d) {
+  return (bits64(a) << 1) == 0 || (bits64(b) << 1) == 0 || (bits64(c) << 1) == 0 ||
+         (bits64(d) << 1) == 0;
+}
+#endif
+
 // ------------------------------------------------------------------ forces
 // hydro_kn_getforceP + getforceQ (hydro_kn_getforce.f90:30-71)
 __device__ __forceinline__ void force_pq(double p, double a1, double a3, double b1, double b3,
@@ -369,14 +388,21 @@ __device__ __forceinline__ void force_pq(double p, double a1, double a3, double 
   fy[2] = fma(p, da, qy.z);
   fy[3] = fma(p, sa, qy.w);
 #else
-  fx[0] = p * (-b3 + b1);
-  fx[1] = p * (b3 + b1);
-  fx[2] = p * (b3 - b1);
-  fx[3] = p * (-b3 - b1);
-  fy[0] = p * (a3 - a1);
-  fy[1] = p * (-a3 - a1);
-  fy[2] = p * (-a3 + a1);
-  fy[3] = p * (a3 + a1);
+  const double db = -b3 + b1, sb = b3 + b1, da = a3 - a1, sa = a3 + a1;
+  fx[0] = p * db;
+  fx[1] = p * sb;
+  fy[0] = p * da;
+  fy[3] = p * sa;
+  fx[2] = negF(fx[0]);
+  fx[3] = negF(fx[1]);
+  fy[2] = negF(fy[0]);
+  fy[1] = negF(fy[3]);
+  if (any_zero(db, sb, da, sa)) {
+    fx[2] = p * (b3 - b1);
+    fx[3] = p * (-b3 - b1);
+    fy[1] = p * (-a3 - a1);
+    fy[2] = p * (-a3 + a1);
+  }
   fx[0] = fx[0] + qx.x;
   fy[0] = fy[0] + qy.x;
   fx[1] = fx[1] + qx.y;
@@ -416,14 +442,21 @@ __device__ void force_sp(double w1, double rho, double cs2, const double* cx, co
     w2 = DIV(c4(spm, j1), w2);
     w2 = w2 - rho;
     w2 = cs2 * w2;
-    lfx[j1][0] = w2 * (w5 - w6);
-    lfx[j1][1] = w2 * (w5 + w6);
-    lfx[j1][2] = w2 * (-w5 + w6);
-    lfx[j1][3] = w2 * (-w5 - w6);
-    lfy[j1][0] = w2 * (-w3 + w4);
-    lfy[j1][1] = w2 * (-w3 - w4);
-    lfy[j1][2] = w2 * (w3 - w4);
-    lfy[j1][3] = w2 * (w3 + w4);
+    const double d = w5 - w6, s = w5 + w6, dy = -w3 + w4, sy = w3 + w4;
+    lfx[j1][0] = w2 * d;
+    lfx[j1][1] = w2 * s;
+    lfy[j1][0] = w2 * dy;
+    lfy[j1][3] = w2 * sy;
+    lfx[j1][2] = negF(lfx[j1][0]);
+    lfx[j1][3] = negF(lfx[j1][1]);
+    lfy[j1][2] = negF(lfy[j1][0]);
+    lfy[j1][1] = negF(lfy[j1][3]);
+    if (any_zero(d, s, dy, sy)) {
+      lfx[j1][2] = w2 * (-w5 + w6);
+      lfx[j1][3] = w2 * (-w5 - w6);
+      lfy[j1][1] = w2 * (-w3 - w4);
+      lfy[j1][2] = w2 * (w3 - w4);
+    }
   }
   double w2 = half(lfx[0][3] + lfx[3][1]);
   double w3 = half(lfx[0][1] + lfx[1][3]);
@@ -1509,6 +1542,11 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
 // joins its faces through shuffles.  One thread per element took its four
 // faces one after another with 676 bytes of spills; the step of a 1,000-element
 // tube took 66.9 us, now 41.6, Sedov 128x128 89.8, now 68.5, 512x512 596, now 581.
+// An edge whose ends move alike -- fluid at rest -- has length 0 in velocity:
+// whatever the limiter says its force is cut (0 <= zerocut) and its viscosity
+// is 0 (or 0 in MAX's first place against a NaN), so it stops there:
+// Sedov 512x512
+// after 60 steps 556 -> 395 us a step, 128x128 67.9 -> 63.9.
 #ifndef BL_EDGE_MINB
 #define BL_EDGE_MINB 7
 #endif
@@ -1522,13 +1560,25 @@ __global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C
     const DevStep* S = el_step<true>(F, iel);
     in = !(halted(S) || S->stop_next);
   }
+  auto ipick = [](const int4& v, int j) {
+    return j == 0 ? v.x : (j == 1 ? v.y : (j == 2 ? v.z : v.w));
+  };
   double ex = 0.0, ey = 0.0, visc = 0.0;
+  double du = 0.0, dv = 0.0, squ = 0.0;
+  int4 n = make_int4(0, 0, 0, 0);
   if (in) {
+    n = L::nodes(F, iel);
+    const int na = ipick(n, is), nn = ipick(n, jn);
+    du = F.ndu[nn] - F.ndu[na];
+    dv = F.ndv[nn] - F.ndv[na];
+    squ = du * du + dv * dv;
+  }
+  if (in && ((bits64(squ) << 1) != 0 || !geF(C.zerocut, 0.0))) {
     // hydro_kn_initeviscosity / limiteviscosity / geteviscosity
     // (hydro_kn_edgeviscosity.f90:30-282).  Face is runs corner is -> is+1;
     // the faces of side s (neighbours across faces s and s+2) are (s+3)&3
     // and s+1.
-    const int4 n = L::nodes(F, iel), nb = L::nbrs(F, iel);
+    const int4 nb = L::nbrs(F, iel);
     const int fcp = L::faces(F, iel);
     const double zc = C.zerocut;
     const double rho0 = F.rho[iel], cs2i = F.cs2[iel];
@@ -1539,11 +1589,7 @@ __global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C
     auto pick = [](const double* v, int j) {
       return j == 0 ? v[0] : (j == 1 ? v[1] : (j == 2 ? v[2] : v[3]));
     };
-    auto ipick = [](const int4& v, int j) {
-      return j == 0 ? v.x : (j == 1 ? v.y : (j == 2 ? v.z : v.w));
-    };
     const double xa = pick(x, is), xb = pick(x, jn), ya = pick(y, is), yb = pick(y, jn);
-    const int na = ipick(n, is), nn = ipick(n, jn);
     const int s = (is & 1) ? 0 : 1;
     const bool first = is == 3 || is == 0;
     const int in1 = ipick(nb, s), in2 = ipick(nb, s + 2);
@@ -1558,10 +1604,9 @@ __global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C
     if (in2 == iel)
       r2 = (__ldg(F.indtype + ipick(n, s + 2)) < 0 &&
             __ldg(F.indtype + ipick(n, (s + 3) & 3)) < 0 && in1 != iel) ? 1.0 : 0.0;
-    double w1 = F.ndu[nn] - F.ndu[na], w2 = F.ndv[nn] - F.ndv[na];
+    double w1 = du, w2 = dv;
     double w3 = xb - xa, w4 = yb - ya;
-    const double du = w1, dv = w2;
-    double den = SQRT(w1 * w1 + w2 * w2);
+    double den = SQRT(squ);
     const double lu = den;
     den = DIV(1.0, maxF_nn(den, zc));
     const double uhat = w1 * den, vhat = w2 * den;

@@ -1,0 +1,45 @@
+"""The edge viscosity of fluid at rest, which the exact build leaves out edge
+by edge: patches of nodes at rest, of zeros of either sign, moving alike and
+moving apart, a cell of infinite density, with and without the zero cut-off.
+Equal to the CPU restatement bit for bit."""
+import numpy as np
+import pytest
+
+from bookleaf_f90_gb300 import Problem, Solver, abi, configs
+
+pytestmark = pytest.mark.gpu
+
+
+def _patches(n, zerocut):
+    p = Problem.from_deck(configs.sedov(n, kappa=0.01, pmerit=0.1))
+    f = p.fields
+    p.config.zerocut = zerocut
+    x, y = f[abi.NDX], f[abi.NDY]
+    top, right = y > 0.5 * y.max(), x > 0.5 * x.max()
+    f[abi.NDU][...] = 0.0
+    f[abi.NDV][...] = 0.0
+    f[abi.NDU][top & ~right] = -0.0
+    f[abi.NDV][(top & ~right) & (np.arange(x.size) % 2 == 0)] = -0.0
+    f[abi.NDU][right & ~top], f[abi.NDV][right & ~top] = 0.3, -0.2
+    apart = right & top
+    f[abi.NDU][apart] = -x[apart] ** 2
+    f[abi.NDV][apart] = 0.5 * x[apart] * y[apart] - y[apart]
+    return p
+
+
+@pytest.mark.parametrize("zerocut", [1e-40, 1e-6, 0.0])
+@pytest.mark.parametrize("n", [5, 12, 33])
+def test_exact_edges_at_rest(n, zerocut):
+    from oracle.oracle import Oracle
+    pg = _patches(n, zerocut)
+    pg.fields[abi.ELDENSITY][n + 1] = np.inf
+    pc = pg.copy()
+    o = Oracle(pc)
+    s = Solver(pg, fp_mode=abi.FP_EXACT)
+    assert s.inf_solver_getdt() == o.getdt(pc.timestep)
+    s.sync_to_host(0)
+    s.close()
+    assert pg.timestep.as_tuple() == pc.timestep.as_tuple()
+    for fid in (abi.ELVISC, abi.CNVISCX, abi.CNVISCY, abi.ELCS2):
+        assert np.array_equal(pg.fields[fid], pc.fields[fid], equal_nan=True), abi.NAMES[fid]
+    assert np.any(pc.fields[abi.ELVISC] > 0.0)
