@@ -1007,7 +1007,20 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_edgevisc(DevFields F, Dev
   }
   if (own) {
     const double rho0 = F.rho[iel];
-    {
+    // four corners of one finite velocity -- fluid at rest: every face's
+    // velocity difference is 0, so its force is cut (0 <= zerocut) and its
+    // viscosity 0, whatever the limiter says.  Sedov 301x301 after 60 steps
+    // 78.5 -> 76.9 us a step, 512x512 174.1 -> 160.6.
+    const long long ub = bits64(u[0]), vb = bits64(v[0]);
+    constexpr long long kExp = 0x7FF0000000000000ll;
+    const bool still = ((ub ^ bits64(u[1])) | (ub ^ bits64(u[2])) | (ub ^ bits64(u[3])) |
+                        (vb ^ bits64(v[1])) | (vb ^ bits64(v[2])) | (vb ^ bits64(v[3]))) == 0 &&
+                       (ub & kExp) != kExp && (vb & kExp) != kExp && zl > (lr)0 && !nanF(rho0);
+    if (still) {
+      F.cnviscx[iel] = make_d4(0.0, 0.0, 0.0, 0.0);
+      F.cnviscy[iel] = make_d4(0.0, 0.0, 0.0, 0.0);
+      F.visc[iel] = 0.0;
+    } else {
       // hydro_kn_initeviscosity / limiteviscosity / geteviscosity
       // (hydro_kn_edgeviscosity.f90:30-282), face by face in the reference's
       // order 3, 1, 0, 2 (the faces of side s are (s+3)&3 and s+1)
