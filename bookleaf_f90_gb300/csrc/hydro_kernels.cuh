@@ -2222,7 +2222,25 @@ __global__ void BL_STATE_BOUNDS(BS) k_lag_state(DevFields F, DevCfg C) {
   const d4 f4x = F.cnfx[iel], f4y = F.cnfy[iel];
   const double fx[4] = {f4x.x, f4x.y, f4x.z, f4x.w};
   const double fy[4] = {f4y.x, f4y.y, f4y.z, f4y.w};
-  const double e = energy_update(e0, m, zc, dt, fx, fy, ub, vb);
+  // no work on fluid at rest, with finite forces: then e0 - 0*dt, which is e0
+  // bit for bit unless that is a zero itself.  Sedov 512x512 after 60
+  // steps: 26.7 -> 23.1 us (exact 42.9 -> 35.0); in motion as before.
+  double e = e0;
+  const long long still = bits64(ub[0]) | bits64(ub[1]) | bits64(ub[2]) | bits64(ub[3]) |
+                          bits64(vb[0]) | bits64(vb[1]) | bits64(vb[2]) | bits64(vb[3]);
+  bool rest = (still << 1) == 0 && (bits64(e0) << 1) != 0;
+  if (rest) {
+    unsigned x = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      x = max(x, (unsigned)(bits64(fx[j]) >> 32) & 0x7ff00000u);
+      x = max(x, (unsigned)(bits64(fy[j]) >> 32) & 0x7ff00000u);
+    }
+    x = max(x, max((unsigned)(bits64(e0) >> 32) & 0x7ff00000u,
+                   (unsigned)(bits64(m) >> 32) & 0x7ff00000u));
+    rest = x != 0x7ff00000u && gtF(zc, 0.0);
+  }
+  if (!rest) e = energy_update(e0, m, zc, dt, fx, fy, ub, vb);
   if (!LOOP || !ale_on(C, S)) {
     double p, cs2;
     eos_pc(C, mat, rho, e, p, cs2);

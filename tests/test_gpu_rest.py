@@ -106,3 +106,22 @@ def test_infinite_pressure_at_rest_is_not_left_out(fp):
     s.sync_to_host(0)
     s.close()
     assert np.isnan(p.fields[abi.ELENERGY][13])
+
+
+@pytest.mark.parametrize("n", [5, 12, 33])
+def test_exact_step_of_cells_at_rest(n):
+    """k_lag_state's energy at rest: bit for bit the restatement's, zero
+    energies of either sign among them."""
+    from oracle.oracle import Oracle
+    pg = _patches(n, 1e-40)
+    e = pg.fields[abi.ELENERGY]
+    e[1], e[n] = 0.0, -0.0
+    pc = pg.copy()
+    o = Oracle(pc)
+    s = Solver(pg, fp_mode=abi.FP_EXACT)
+    for _ in range(3):
+        assert s.step() == o.step(pc.timestep) == 0
+    s.sync_to_host(0)
+    s.close()
+    for fid in (abi.ELENERGY, abi.ELDENSITY, abi.ELPRESSURE, abi.NDU, abi.NDV, abi.NDX):
+        assert np.array_equal(pg.fields[fid], pc.fields[fid]), abi.NAMES[fid]
