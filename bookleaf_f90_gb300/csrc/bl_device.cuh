@@ -119,7 +119,9 @@ struct DevFields {
   // with its nodes, elements and the edges that continue it, and each
   // element's four slots
   int nslot;
-  int geom_x;                // a1..b3 may not be those of the node positions
+  int geom_x;                // a1..b3 or vol are not those of the node positions
+                             // (k_check_geometry): kernels that may take either
+                             // then take each from where the reference does
   const int4* es_n;          // [nslot] nodes a, b, element, element across
   const int4* es_q;          // [nslot] continuing edges' nodes, or codes < 0
   const uint4* eref;         // [nel] 2*slot + (1: run the other way) of each face

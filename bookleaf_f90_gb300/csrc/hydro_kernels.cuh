@@ -571,13 +571,14 @@ struct DevLayout {
 // sides of geometry_kn_dlm or _dln), or -1 for a zdtnotreg region (the
 // reference's HUGE candidate); it does not depend on the viscosity.
 // corners(x, y) brings the corner positions where they are needed.
-template <class L = DevLayout, class Q>
+// (POS: the kernels' form for coefficients that may not be the positions')
+template <class L = DevLayout, bool POS = false, class Q>
 __device__ __forceinline__ double getdt_cfl_len(const DevFields& F, const DevCfg& C, int iel,
                                                 Q corners) {
   const int ireg = L::reg(F, iel);
   if (__ldg(C.zdtnotreg + ireg)) return -1.0;
 #if BL_MIXED
-  if (!__ldg(C.zmidlength + ireg))
+  if (!POS && !__ldg(C.zmidlength + ireg))
     return from_lr(min_dln_iso<lr>(corners, lr_cut(C.zcut), to_lr(F.a1[iel]), to_lr(F.a2[iel]),
                                    to_lr(F.a3[iel]), to_lr(F.b1[iel]), to_lr(F.b2[iel]),
                                    to_lr(F.b3[iel])));
@@ -585,7 +586,10 @@ __device__ __forceinline__ double getdt_cfl_len(const DevFields& F, const DevCfg
   double x[4], y[4];
   corners(x, y);
 #if BL_MIXED
-  return min_dlm(x, y);
+  if (!POS || __ldg(C.zmidlength + ireg)) return min_dlm(x, y);
+  const Iso g = getiso(x, y);
+  return from_lr(min_dln_iso<lr>(corners, lr_cut(C.zcut), to_lr(g.a1), to_lr(g.a2), to_lr(g.a3),
+                                 to_lr(g.b1), to_lr(g.b2), to_lr(g.b3)));
 #else
   return __ldg(C.zmidlength + ireg) ? min_dlm(x, y) : min_dln(x, y, C.zcut);
 #endif
@@ -646,12 +650,12 @@ __device__ __forceinline__ void getdt_cfl(const DevFields& F, int iel, double le
 
 // hydro_dr_getcs2, then the element's hydro_kn_getdtcfl and getdtdiv
 // candidates
-template <class L = DevLayout, class Q>
+template <class L = DevLayout, bool POS = false, class Q>
 __device__ __forceinline__ void getdt_tail(const DevFields& F, const DevCfg& C, int iel,
                                            Q corners, const double* u, const double* v,
                                            double visc, double& cflv, int& cfli, double& divv,
                                            int& divi) {
-  getdt_cfl(F, iel, getdt_cfl_len<L>(F, C, iel, corners), visc, cflv, cfli);
+  getdt_cfl(F, iel, getdt_cfl_len<L, POS>(F, C, iel, corners), visc, cflv, cfli);
   getdt_div(F, iel, u, v, divv, divi);
 }
 
@@ -944,7 +948,7 @@ __device__ __forceinline__ lr nb_ratio(const FaceQ& f, lr ddx, lr ddy, lr ddu, l
 // The FP64 build's form, one thread per edge of the mesh (k_edge), would be
 // no slower here, but FP32 rounds each of an edge's two sides its own way: it
 // would change results in the seventh digit, so the element form stays.
-template <int BS, bool BATCH>
+template <int BS, bool BATCH, bool POS>
 __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_edgevisc(DevFields F, DevCfg C) {
   const int t = threadIdx.x;
   const int iel = (int)blockIdx.x * (BS - 2) + t - 1;
@@ -1031,7 +1035,14 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_edgevisc(DevFields F, Dev
       // the vector from an edge's midpoint to the centroid is (a3,b3),
       // (-a1,-b1), (-a3,-b3), (a1,b1) for faces 0..3 (corners written as
       // s -+ a1 +- a2 -+ a3, exact in real arithmetic)
-      const lr ga1 = to_lr(F.a1[iel]), ga3 = to_lr(F.a3[iel]), gb1 = to_lr(F.b1[iel]), gb3 = to_lr(F.b3[iel]);
+      double ca1, ca3, cb1, cb3;
+      if (POS) {
+        const Iso g = getiso(x, y);
+        ca1 = g.a1, ca3 = g.a3, cb1 = g.b1, cb3 = g.b3;
+      } else {
+        ca1 = F.a1[iel], ca3 = F.a3[iel], cb1 = F.b1[iel], cb3 = F.b3[iel];
+      }
+      const lr ga1 = to_lr(ca1), ga3 = to_lr(ca3), gb1 = to_lr(cb1), gb3 = to_lr(cb3);
       // |c|^2 of faces 1,3 and of faces 0,2 (only the cut test uses it)
       const lr c1sq = ga1 * ga1 + gb1 * gb1, c3sq = ga3 * ga3 + gb3 * gb3;
       // max over faces of edv * |du|; the reference's max of
@@ -1171,7 +1182,7 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_edgevisc(DevFields F, Dev
 // element): the positions are brought only for the regions and faces that
 // need them, and a block takes several tiles.  (8, 10 and 12 blocks per SM,
 // with the registers that leaves, are slower.)
-template <int BS, bool BATCH>
+template <int BS, bool BATCH, bool POS>
 __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg C) {
   DevStep* S = F.step;
   int blk0 = 0, nblk = (int)gridDim.x, el0 = 0, el1 = F.nel;
@@ -1212,7 +1223,7 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
         y[j] = F.ndy[n[j]];
       }
     };
-    getdt_tail(F, C, iel, corners, u, v, F.visc[iel], cflv, cfli, divv, divi);
+    getdt_tail<DevLayout, POS>(F, C, iel, corners, u, v, F.visc[iel], cflv, cfli, divv, divi);
   }
   getdt_finish<BS, BATCH>(F, C, S, cflv, cfli, divv, divi, blk0, nblk, el0, I);
 }
@@ -1445,8 +1456,8 @@ __device__ __forceinline__ double cfl_candidate(const DevFields& F, const DevCfg
 
 // One thread per element: its corner viscosity forces and viscosity from
 // its edges, elcs2 + elvisc, and its CFL and divergence candidates; then
-// the dt reduction.
-template <int BS, bool BATCH>
+// the dt reduction.  (POS: DevFields::geom_x)
+template <int BS, bool BATCH, bool POS>
 __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg C) {
   // the mesh of this block: the context's, or in a batch the block's own
   // (its blocks [blk0, blk0 + nblk), elements [el0, el1))
@@ -1481,13 +1492,26 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
     const unsigned er[4] = {er4.x, er4.y, er4.z, er4.w};
     double visc = 0.0;
     double du[4], dv[4], sq[4], W[4], edx[4], edy[4];
-    const double a1 = F.a1[iel], a2 = F.a2[iel], a3 = F.a3[iel];
-    const double b1 = F.b1[iel], b2 = F.b2[iel], b3 = F.b3[iel];
+    double a1 = F.a1[iel], a2, a3 = F.a3[iel], b1 = F.b1[iel], b2, b3 = F.b3[iel];
     const double vol = F.vol[iel], rho = F.rho[iel], cs2 = F.cs2[iel];
+    // the divergence limit's coefficients are the stored ones in any case
+    const double da1 = a1, da3 = a3, db1 = b1, db3 = b3;
     const int ireg = __ldg(F.ielreg + iel);
     const int notdt = __ldg(C.zdtnotreg + ireg), mid = __ldg(C.zmidlength + ireg);
     {
-      const double cross = quarter(vol);
+      double cross;
+      if (POS) {
+        const int4 n = __ldg(F.ielnd + iel);
+        const double x[4] = {F.ndx[n.x], F.ndx[n.y], F.ndx[n.z], F.ndx[n.w]};
+        const double y[4] = {F.ndy[n.x], F.ndy[n.y], F.ndy[n.z], F.ndy[n.w]};
+        const Iso g = getiso(x, y);
+        a1 = g.a1, a2 = g.a2, a3 = g.a3, b1 = g.b1, b2 = g.b2, b3 = g.b3;
+        cross = g.cross;
+      } else {
+        a2 = F.a2[iel];
+        b2 = F.b2[iel];
+        cross = quarter(vol);
+      }
       const double t1 = a1 * b2 - a2 * b1, t3 = a3 * b2 - a2 * b3;
       W[0] = cross + t3;
       W[1] = cross + t1;
@@ -1532,8 +1556,8 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
     const double cs2v = signal_speed(F, iel, cs2, visc);
     cfl_min(cflv, cfli, cfl_candidate(F, C, iel, W, sq, a1, a2, a3, b1, b2, b3, cs2v, notdt, mid),
             iel);
-    const double w = b1 * (du[3] - du[1]) + b3 * (du[0] - du[2]) - a1 * (dv[3] - dv[1]) -
-                     a3 * (dv[0] - dv[2]);
+    const double w = db1 * (du[3] - du[1]) + db3 * (du[0] - du[2]) - da1 * (dv[3] - dv[1]) -
+                     da3 * (dv[0] - dv[2]);
     const double dd = DIV(absF(w), vol);
     if (gt_nn(dd, divv)) {
       divv = dd;
@@ -1769,9 +1793,10 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
 // 512x512 108 -> 90 us (FP64 pipe 79 % busy over the SMs' active cycles, the
 // divide chains' latency the rest; 3, 5 and 6 blocks per SM and blocks of 64
 // and 256 threads are slower or equal), 42 -> 39 us at 90,000 elements.
-// Where the coefficients may not be those of the positions (F.geom_x: a2 or
-// b2 not registered, or positions uploaded on their own) the half-step
-// geometry is formed from the corners.
+// POS: where the coefficients or volumes are not those of the positions
+// (DevFields::geom_x), the half-step geometry and the sub-zonal pressures are
+// formed from the corners; the pressure force keeps the stored coefficients,
+// as the reference's does.
 struct SubZone {
   double q[4];  // sub-zonal densities spmass_j / V_j
 };
@@ -1806,7 +1831,7 @@ __device__ __forceinline__ void corner_forces(double d, double s, double c2, con
   }
 }
 
-template <int BS, bool BATCH>
+template <int BS, bool BATCH, bool POS>
 __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, DevCfg C) {
   const int iel = blockIdx.x * BS + threadIdx.x;
   if (iel >= F.nel) return;
@@ -1862,21 +1887,37 @@ __global__ void __launch_bounds__(BS, BL_FORCE_MINB) k_lag_force(DevFields F, De
     const double Dv = (d * u02 + s * u13) - (dy * v02 + sy * v13);
     work = p0 * Dv + qx.x * u[0] + qy.x * v[0] + qx.y * u[1] + qy.y * v[1] + qx.z * u[2] +
            qy.z * v[2] + qx.w * u[3] + qy.w * v[3];
-    if (C.zsp) {
-      const double t1 = a1 * b2 - a2 * b1, t3 = a3 * b2 - a2 * b3;
-      const SubZone z = sub_zone(quarter(F.vol[iel]), t1 + t3, t3 - t1, F.spmass[iel]);
+    auto sub_zone_work = [&](const SubZone& z, double d, double s, double dy, double sy, double a2,
+                             double b2, double Dv) {
       const double b22 = twice(b2), a22 = twice(a2);
       const double B = (d * hu - b22 * u13) - (dy * hv - a22 * v13);
       const double D = (s * hu + b22 * u02) - (sy * hv + a22 * v02);
       const double sum = fma(-4.0, F.rho[iel], (z.q[0] + z.q[2]) + (z.q[1] + z.q[3]));
       const double w = fma(twice(Dv), sum, fma(B, z.q[0] - z.q[2], -(D * (z.q[1] - z.q[3]))));
-      work = fma(ldexpF<-3>(pm) * F.cs2v[iel], w, work);
+      return fma(ldexpF<-3>(pm) * F.cs2v[iel], w, work);
+    };
+    if (C.zsp && !POS) {
+      const double t1 = a1 * b2 - a2 * b1, t3 = a3 * b2 - a2 * b3;
+      const SubZone z = sub_zone(quarter(F.vol[iel]), t1 + t3, t3 - t1, F.spmass[iel]);
+      work = sub_zone_work(z, d, s, dy, sy, a2, b2, Dv);
+    } else if (C.zsp) {
+      double x[4], y[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        x[j] = F.ndx[n[j]];
+        y[j] = F.ndy[n[j]];
+      }
+      const Iso g = getiso(x, y);
+      const SubZone z = sub_zone(g.cross, g.ts, g.td, F.spmass[iel]);
+      const double gd = g.b1 - g.b3, gs = g.b1 + g.b3, gdy = g.a1 - g.a3, gsy = g.a1 + g.a3;
+      work = sub_zone_work(z, gd, gs, gdy, gsy, g.a2, g.b2,
+                           (gd * u02 + gs * u13) - (gdy * v02 + gsy * v13));
     }
   }
   // ---- geometry at the half step (geometry_kn_getvertex with 0.5*dt,
   // geometry_dr_getgeometry), density
   Iso g;
-  if (!F.geom_x) {
+  if (!POS) {
     const double r = quarter(hdt);
     g.a1 = fma(r, u13 - u02, a1);
     g.a2 = fma(r, hu, a2);
@@ -2474,18 +2515,42 @@ int getdt_launches(const DevCfg& C) {
   return C.ztq ? 1 : 2;
 #endif
 }
-void launch_getdt(const DevFields& F, const DevCfg& C, cudaStream_t s) {
+// (the kernels' POS forms where DevFields::geom_x says so; the exact build
+// always takes the positions)
+template <bool BATCH>
+static void getdt_kernels(const DevFields& F, const DevCfg& C, int grid, cudaStream_t s) {
 #if BL_MIXED
-  if (!C.ztq) k_edgevisc<BS_DT, false><<<edge_grid(F.nel), BS_DT, 0, s>>>(F, C);
+  if (!C.ztq) {
+    if (F.geom_x) k_edgevisc<BS_DT, BATCH, true><<<edge_grid(F.nel), BS_DT, 0, s>>>(F, C);
+    else k_edgevisc<BS_DT, BATCH, false><<<edge_grid(F.nel), BS_DT, 0, s>>>(F, C);
+  }
 #elif BL_FAST_ALGEBRA
-  k_edge<BS_ED, false><<<edge_grid(F.nslot), BS_ED, 0, s>>>(F, C);
+  k_edge<BS_ED, BATCH><<<edge_grid(F.nslot), BS_ED, 0, s>>>(F, C);
 #else
-  if (!C.ztq) k_edge<BS_ED, false><<<face_grid(F.nel), BS_ED, 0, s>>>(F, C);
+  if (!C.ztq) k_edge<BS_ED, BATCH><<<face_grid(F.nel), BS_ED, 0, s>>>(F, C);
 #endif
-  k_getdt<BS_DT, false><<<getdt_grid(F.nel), BS_DT, 0, s>>>(F, C);
+#if BL_FAST_ALGEBRA
+  if (F.geom_x) k_getdt<BS_DT, BATCH, true><<<grid, BS_DT, 0, s>>>(F, C);
+  else k_getdt<BS_DT, BATCH, false><<<grid, BS_DT, 0, s>>>(F, C);
+#else
+  k_getdt<BS_DT, BATCH><<<grid, BS_DT, 0, s>>>(F, C);
+#endif
+}
+template <bool BATCH>
+static void force_kernel(const DevFields& F, const DevCfg& C, cudaStream_t s) {
+  const int g = (F.nel + BS_EL - 1) / BS_EL;
+#if BL_FAST_ALGEBRA
+  if (F.geom_x) k_lag_force<BS_EL, BATCH, true><<<g, BS_EL, 0, s>>>(F, C);
+  else k_lag_force<BS_EL, BATCH, false><<<g, BS_EL, 0, s>>>(F, C);
+#else
+  k_lag_force<BS_EL, BATCH><<<g, BS_EL, 0, s>>>(F, C);
+#endif
+}
+void launch_getdt(const DevFields& F, const DevCfg& C, cudaStream_t s) {
+  getdt_kernels<false>(F, C, getdt_grid(F.nel), s);
 }
 void launch_lag_force(const DevFields& F, const DevCfg& C, cudaStream_t s) {
-  k_lag_force<BS_EL, false><<<(F.nel + BS_EL - 1) / BS_EL, BS_EL, 0, s>>>(F, C);
+  force_kernel<false>(F, C, s);
 }
 void launch_lag_accel(const DevFields& F, const DevCfg& C, cudaStream_t s) {
   k_lag_accel<BS_ND, false><<<(F.nnd + BS_ND - 1) / BS_ND, BS_ND, 0, s>>>(F, C);
@@ -2517,17 +2582,10 @@ void launch_mix_closure_batch(const DevFields& F, const DevCfg& C, cudaStream_t 
 // a batch of meshes: k_getdt over each mesh's own blocks, the rest over all
 // elements or nodes, each reading the step header of its mesh
 void launch_getdt_batch(const DevFields& F, const DevCfg& C, cudaStream_t s) {
-#if BL_MIXED
-  if (!C.ztq) k_edgevisc<BS_DT, true><<<edge_grid(F.nel), BS_DT, 0, s>>>(F, C);
-#elif BL_FAST_ALGEBRA
-  k_edge<BS_ED, true><<<edge_grid(F.nslot), BS_ED, 0, s>>>(F, C);
-#else
-  if (!C.ztq) k_edge<BS_ED, true><<<face_grid(F.nel), BS_ED, 0, s>>>(F, C);
-#endif
-  k_getdt<BS_DT, true><<<F.nblk_batch, BS_DT, 0, s>>>(F, C);
+  getdt_kernels<true>(F, C, F.nblk_batch, s);
 }
 void launch_lag_force_batch(const DevFields& F, const DevCfg& C, cudaStream_t s) {
-  k_lag_force<BS_EL, true><<<(F.nel + BS_EL - 1) / BS_EL, BS_EL, 0, s>>>(F, C);
+  force_kernel<true>(F, C, s);
 }
 void launch_lag_accel_batch(const DevFields& F, const DevCfg& C, cudaStream_t s) {
   // block size chosen by the batch's autotuner (128, 256 or 512)

@@ -1,0 +1,164 @@
+"""Node positions, element coefficients and volumes that do not agree: a host
+may move its nodes, or change a coefficient or a volume, and upload that
+field alone, the whole state, or have it so when the context is made.  The
+time step, the viscosity, the half-step geometry and the sub-zonal volumes
+come from the positions; the pressure force and the divergence limit from the
+coefficients and volumes (geometry_dr_getgeometry has not run since).
+
+Tolerance: the fast build at most 1e3 roundings (1.1e-16 each), amplified at
+most 1e2 times by differences: 1e-10 relative L1, and 1e-11 on the time step.
+The mixed build, whose viscosity and CFL lengths are FP32, some hundred
+roundings of 6e-8: 1e-5."""
+import numpy as np
+import pytest
+
+from bookleaf_f90_gb300 import BatchSolver, Problem, Solver, abi, configs
+
+pytestmark = pytest.mark.gpu
+
+BLAST = configs.sedov(12, kappa=0.01, pmerit=0.1)
+DECKS = {
+    "all_forces": BLAST,
+    "polar": configs.noh_polar(17, 9),
+    "midlength": BLAST.replace("cvisc2=0.75\n", "cvisc2=0.75\n zmidlength(1)=.TRUE.\n"),
+    "short_faces": BLAST.replace("&INDICATORS", "&CUTOFF\n zcut=1.0e-1\n/\n&INDICATORS", 1),
+    "mixed_cells": configs.sod_multimaterial(24, 6),
+}
+BUILDS = {"fast": (abi.FP_FAST, 1e-10, 1e-11), "mixed": (abi.FP_MIXED, 1e-5, 1e-5)}
+COEFFICIENTS = [abi.A1, abi.A2, abi.A3, abi.B1, abi.B2, abi.B3]
+
+
+def _moving(deck):
+    """A problem whose fluid all moves, with one step behind it, and a next
+    time step that only the CFL and divergence limits bound."""
+    from oracle.oracle import Oracle
+    p = Problem.from_deck(deck)
+    f = p.fields
+    p.config.dt_g, p.config.dt_max = 1e9, 1e9
+    x, y = f[abi.NDX] / f[abi.NDX].max(), f[abi.NDY] / f[abi.NDY].max()
+    f[abi.NDU] -= 0.3 * x * x - 0.1 * x * y
+    f[abi.NDV] += 0.2 * x * y - 0.25 * y
+    f[abi.ELENERGY] += 0.05
+    assert Oracle(p).step(p.timestep) == 0
+    return p
+
+
+def _change(p, what):
+    """Change p's host fields; the ids that changed."""
+    f = p.fields
+    rng = np.random.default_rng(11)
+    if what == "positions":
+        nd = f[abi.IELND] - 1
+        h = np.sqrt(np.min(f[abi.ELVOLUME]))
+        for fid, cn in ((abi.NDX, abi.CNX), (abi.NDY, abi.CNY)):
+            f[fid] += 0.04 * h * rng.uniform(-1.0, 1.0, p.nnd) * (f[abi.INDTYPE] > 0)
+            f[cn][...] = f[fid][nd]
+        return [abi.NDX, abi.NDY]
+    if what == "volumes":
+        f[abi.ELVOLUME] *= 1.0 + 0.05 * rng.uniform(-1.0, 1.0, p.nel)
+        return [abi.ELVOLUME]
+    for fid in COEFFICIENTS:
+        f[fid] *= 1.0 + 0.03 * rng.uniform(-1.0, 1.0, p.nel)
+    # (the components' are gathers of the elements', as cnx is of ndx)
+    for m in range(p.sizes.nmx):
+        k, e = f[abi.IMXFCP][m] - 1, f[abi.IMXEL][m] - 1
+        for cp, el in ((abi.CPA1, abi.A1), (abi.CPA3, abi.A3), (abi.CPB1, abi.B1),
+                       (abi.CPB3, abi.B3)):
+            f[cp][k:k + f[abi.IMXNCP][m]] = f[el][e]
+    return COEFFICIENTS
+
+
+def _off(pg, pc, sets, tol):
+    kinetic = 0.5 * np.sum(pc.fields[abi.NDU] ** 2 + pc.fields[abi.NDV] ** 2)
+    for ids in sets:
+        off = sum(np.sum(np.abs(pg.fields[f] - pc.fields[f])) for f in ids)
+        size = sum(np.sum(np.abs(pc.fields[f])) for f in ids)
+        if ids[0] in (abi.ELENERGY, abi.ELPRESSURE):
+            size += kinetic
+        assert off <= tol * size, (abi.NAMES[ids[0]], off, size)
+
+
+STEP = ((abi.ELDENSITY,), (abi.ELENERGY,), (abi.ELPRESSURE,), (abi.ELVOLUME,),
+        (abi.NDU, abi.NDV), (abi.NDX, abi.NDY))
+
+
+@pytest.mark.parametrize("build", sorted(BUILDS))
+@pytest.mark.parametrize("how", ["made", "whole", "alone"])
+@pytest.mark.parametrize("what", ["positions", "volumes", "coefficients"])
+@pytest.mark.parametrize("name", sorted(DECKS))
+def test_called_step(name, what, how, build):
+    from oracle.oracle import Oracle
+    if name == "mixed_cells" and build == "mixed":
+        pytest.skip("a smooth flow's limiter cancels more than FP32's digits allow for here")
+    fp, tol, tdt = BUILDS[build]
+    pc = _moving(DECKS[name])
+    before = pc.copy()
+    ids = _change(pc, what)
+    pg = pc.copy() if how == "made" else before
+    s = Solver(pg, fp_mode=fp)
+    if how != "made":
+        for f in pg.fields:
+            pg.fields[f][...] = pc.fields[f]
+        for f in [0] if how == "whole" else ids:
+            s.sync_to_device(f)
+    o = Oracle(pc)
+    assert s.inf_solver_getdt() == o.getdt(pc.timestep) == 0
+    assert abs(pg.timestep.dt - pc.timestep.dt) <= tdt * pc.timestep.dt
+    assert pg.timestep.idtel == pc.timestep.idtel
+    s.sync_to_host(0)
+    _off(pg, pc, ((abi.ELVISC,), (abi.ELCS2,), (abi.CNVISCX, abi.CNVISCY)), tol)
+    assert s.inf_solver_lagstep() == o.lagstep(pc.timestep) == 0
+    s.sync_to_host(0)
+    s.close()
+    _off(pg, pc, STEP, tol)
+
+
+@pytest.mark.parametrize("build", sorted(BUILDS))
+@pytest.mark.parametrize("name", ["all_forces", "polar"])
+def test_coefficients_a2_b2_not_registered(name, build):
+    from oracle.oracle import Oracle
+    fp, tol, tdt = BUILDS[build]
+    pc = _moving(DECKS[name])
+    pg = pc.copy()
+    del pg.fields[abi.A2], pg.fields[abi.B2]
+    s = Solver(pg, fp_mode=fp)
+    o = Oracle(pc)
+    assert s.step() == o.step(pc.timestep) == 0
+    assert abs(pg.timestep.dt - pc.timestep.dt) <= tdt * pc.timestep.dt
+    s.sync_to_host(0)
+    s.close()
+    _off(pg, pc, STEP, tol)
+
+
+@pytest.mark.parametrize("build", sorted(BUILDS))
+def test_device_loops(build):
+    """The loops' kernels, of one mesh and of a batch: a run, moved nodes, and
+    the next step, whose graph and arguments are those of the moved state."""
+    from oracle.oracle import Oracle
+    fp, tol, tdt = BUILDS[build]
+    decks = [DECKS["all_forces"], configs.sedov(7, kappa=0.01, pmerit=0.1)]
+    base = [_moving(d) for d in decks]
+    one, batch = base[0].copy(), [p.copy() for p in base]
+    s, b = Solver(one, fp_mode=fp), BatchSolver(batch, fp_mode=fp)
+    assert s.run(max_steps=1, history=False)[0] == 0
+    assert b.run(max_steps=1)[0] == 0
+    for p in base:
+        _change(p, "positions")
+    for p, q in zip([one] + batch, [base[0]] + base):
+        for f in p.fields:
+            p.fields[f][...] = q.fields[f]
+        p.timestep = q.timestep.copy()
+    s.timestep = one.timestep
+    s.sync_to_device(0)
+    assert b.sync_to_device(0) == 0
+    assert s.run(max_steps=1, history=False)[0] == 0
+    assert b.run(max_steps=1)[0] == 0
+    s.sync_to_host(0)
+    assert b.sync_to_host(0) == 0
+    s.close()
+    b.close()
+    for p in base:
+        assert Oracle(p).step(p.timestep) == 0
+    for p, q in zip([one] + batch, [base[0]] + base):
+        assert abs(p.timestep.dt - q.timestep.dt) <= tdt * q.timestep.dt
+        _off(p, q, STEP, tol)
