@@ -1298,9 +1298,10 @@ static __device__ __noinline__ double limiter_general(double du, double dv, doub
 // holds while the squares and products keep clear of the range's ends and
 // of zerocut (tested on their exponents: lengths from 2^-40 to 2^40,
 // velocity differences from 2^-80 to 2^80, zerocut at most 2^-132; the
-// default is 1e-40); other operands take limiter_general.  An edge whose
-// velocity difference is at most zerocut gives no viscosity and skips the
-// rest, as whole warps of still fluid do.
+// default is 1e-40); other operands take limiter_general, among them the
+// edges whose velocity difference is at most zerocut: their force is cut,
+// their viscosity is not.  An edge without a difference has neither and skips
+// the rest, as whole warps of still fluid do.
 // Per edge it leaves (du, dv, E, EL), E = edge coefficient / |U| (0 where
 // the reference cuts the edge) and EL = edge coefficient * |U|, and |D|^2.
 #ifndef BL_EDGE_MINB
@@ -1351,8 +1352,8 @@ __global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C
   if (!(in && t > 0 && t < BS - 1)) return;
   const double squ = fma(d.dv, d.dv, d.du * d.du), sqx = fma(d.dy, d.dy, d.dx * d.dx);
   double E = 0.0, EL = 0.0;
-  const double lu = SQRT(squ);
-  if (!C.ztq && !le_nn(lu, zc)) {
+  if (!C.ztq && (bits64(squ) << 1) != 0) {
+    const double lu = SQRT(squ);
     const double cs = SQRT(half(F.cs2[n.z] + F.cs2[n.w]));
     auto dots = [&](int code, int node, int beside, double& P, double& Q) {
       if (code == kEndAdjacent) {
@@ -1385,7 +1386,7 @@ __global__ void __launch_bounds__(BS, BL_EDGE_MINB) k_edge(DevFields F, DevCfg C
       const EndD o1 = q.x >= 0 || q.x == kEndAdjacent ? diff(q.x, q.y, t - 1) : none;
       const EndD o2 = q.z >= 0 || q.z == kEndAdjacent ? diff(q.z, q.w, t + 1) : none;
       lim = limiter_general(d.du, d.dv, d.dx, d.dy, q.x, o1, q.z, o2, zc);
-      cut = le_nn(SQRT(sqx), zc);
+      cut = le_nn(lu, zc) || le_nn(SQRT(sqx), zc);
     }
     const double edv = half(1.0 - lim) *
                        ((F.rho[n.z] + F.rho[n.w]) * fma(C.cvisc2, lu, C.cvisc1 * cs));
