@@ -91,16 +91,23 @@ __device__ __forceinline__ double grad_f32(double A, double B, double mA, double
 #endif
 
 #if BL_FAST_ALGEBRA && !BL_MIXED
+// neither infinite nor a NaN; that and above zero
+__device__ __forceinline__ bool finiteF(double x) {
+  return ((unsigned)(bits64(x) >> 32) & 0x7ff00000u) != 0x7ff00000u;
+}
+__device__ __forceinline__ bool positiveF(double x) {
+  return (unsigned long long)bits64(x) - 1 < 0x7fefffffffffffffull;
+}
 // -1, 0 or 1 for a * b below, near (within 2^-18) or above c * d, from the
-// leading 21 bits and the exponents, on the integer pipe; 0 also for zero,
-// subnormal, infinite and NaN operands.  Signs are ignored.
+// leading 21 bits and the exponents, on the integer pipe; 0 also for zero and
+// subnormal operands.  Signs are ignored, no operand is infinite or a NaN.
 __device__ __forceinline__ int order_products(double a, double b, double c, double d) {
   const unsigned ha = (unsigned)(bits64(a) >> 32) & 0x7fffffffu;
   const unsigned hb = (unsigned)(bits64(b) >> 32) & 0x7fffffffu;
   const unsigned hc = (unsigned)(bits64(c) >> 32) & 0x7fffffffu;
   const unsigned hd = (unsigned)(bits64(d) >> 32) & 0x7fffffffu;
-  const unsigned lo = 0x00100000u, n = 0x7fe00000u;  // a normal number: hi - lo < n
-  if (ha - lo >= n || hb - lo >= n || hc - lo >= n || hd - lo >= n) return 0;
+  const unsigned lo = 0x00100000u;  // a normal number's at least
+  if (ha < lo || hb < lo || hc < lo || hd < lo) return 0;
   const int e = (int)(ha >> 20) + (int)(hb >> 20) - (int)(hc >> 20) - (int)(hd >> 20);
   if (e > 2 || e < -2) return e > 0 ? 1 : -1;
   const unsigned long long p =
@@ -122,7 +129,15 @@ __device__ __forceinline__ int order_products(double a, double b, double c, doub
 // smaller of those two quotients, and which one that is shows in the
 // products A mB and B mA: one divide, no product in the FP64 pipe, where
 // the three candidates took three divides and seven operations.  (Two
-// divides when the products are too near to tell.)
+// divides when the products are too near to tell.)  Masses of other signs,
+// infinities and NaN take the three candidates.
+__device__ __forceinline__ double slope_of_three(double A, double B, double mA, double mB,
+                                                 double S) {
+  const double w8 = DIV(A * mB * mB + B * mA * mA, mA * mB * (mA + mB));
+  double grad = sign_of(minF(minF(absF(w8), DIV(absF(A), mA)), DIV(absF(B), mB)), S);
+  if (prod_le0(A, B)) grad = 0.0;
+  return grad;
+}
 __device__ __forceinline__ double limited_slope(double A, double B, double mA, double mB,
                                                 double S) {
 #if BL_MIXED
@@ -130,56 +145,53 @@ __device__ __forceinline__ double limited_slope(double A, double B, double mA, d
 #else
 #if BL_FAST_ALGEBRA
   if (prod_le0(A, B)) return 0.0;
-  if (bits64(mA) > 0 && bits64(mB) > 0) {
+  if (finiteF(A) && finiteF(B) && positiveF(mA) && positiveF(mB)) {
     const int o = order_products(A, mB, B, mA);
     const double q = DIV(absF(o > 0 ? B : A), o > 0 ? mB : mA);
     return signF(o == 0 ? minF_nn(q, DIV(absF(B), mB)) : q, S);
   }
 #endif
-  const double w8 = DIV(A * mB * mB + B * mA * mA, mA * mB * (mA + mB));
-  double grad = sign_of(minF(minF(absF(w8), DIV(absF(A), mA)), DIV(absF(B), mB)), S);
-  if (prod_le0(A, B)) grad = 0.0;
-  return grad;
+  return slope_of_three(A, B, mA, mB, S);
 #endif
 }
 
 // The limited face flux of ale_kn_fluxelvl for the pair (i1, i2=i1+2),
 // returning (fcflux(i1), fcflux(i2)) (ale_kn_advectors.f90:48-78).
+// Fast build: where nothing leaves through a face its flux is 0 without the
+// arithmetic -- unless that would be 0 times an infinity or a NaN, which the
+// neighbour has to meet.
 __device__ __forceinline__ void elvl_pair(int i1, const int* nb, const int* fc,
                                           const d4* cnbasis, const double* own_b,
                                           double r1, double r2, const double* elvar,
                                           double rv, double& o1, double& o2) {
   const int i2 = i1 + 2;
+  const int iel1 = nb[i1], iel2 = nb[i2];
+  const double w1 = rv - elvar[iel2], w2 = elvar[iel1] - rv;
+  const double r3 = own_b[i2] + own_b[(i2 + 1) & 3], r4 = own_b[i1] + own_b[i1 + 1];
 #if BL_FAST_ALGEBRA && !BL_MIXED
-  // nothing leaves through either face (fluid at rest)
-  if (((unsigned long long)(bits64(r1) | bits64(r2)) << 1) == 0) {
+  // nothing leaves through either face (fluid at rest), and no slope
+  const bool z1 = (bits64(r1) << 1) == 0, z2 = (bits64(r2) << 1) == 0;
+  if (z1 && z2 && prod_le0(w1, w2) && finiteF(rv) && finiteF(r3) && finiteF(r4)) {
     o1 = o2 = 0.0;
     return;
   }
 #endif
-  const int iel2 = nb[i2];
-  int j2 = fc[i2];
-  double r3 = own_b[i2] + own_b[(i2 + 1) & 3];
-  double w5 = r3 + cget(cnbasis, iel2, j2) + cget(cnbasis, iel2, (j2 + 1) & 3);
-  const int iel1 = nb[i1];
-  j2 = fc[i1];
-  double r4 = own_b[i1] + own_b[i1 + 1];
-  double w6 = r4 + cget(cnbasis, iel1, j2) + cget(cnbasis, iel1, (j2 + 1) & 3);
-  double w1 = rv - elvar[iel2];
-  double w2 = elvar[iel1] - rv;
+  const int f1 = fc[i1], f2 = fc[i2];
+  const double w5 = r3 + cget(cnbasis, iel2, f2) + cget(cnbasis, iel2, (f2 + 1) & 3);
+  const double w6 = r4 + cget(cnbasis, iel1, f1) + cget(cnbasis, iel1, (f1 + 1) & 3);
   const double grad = limited_slope(w1, w2, w5, w6, w2);
 #if BL_FAST_ALGEBRA && !BL_MIXED
   // flow through the pair leaves through one face; the other's flux is 0
-  const bool z1 = (bits64(r1) << 1) == 0, z2 = (bits64(r2) << 1) == 0;
-  const double r = z1 ? r2 : r1;
-  const double o = r * fma(z1 ? negF(grad) : grad, (z1 ? r4 : r3) - half(r), rv);
-  o1 = z1 ? 0.0 : o;
-  o2 = z1 ? o : 0.0;
-  if (!z1 && !z2) o2 = r2 * fma(negF(grad), r4 - half(r2), rv);
-#else
+  if ((z1 || z2) && finiteF(grad) && finiteF(rv) && finiteF(r3) && finiteF(r4)) {
+    const double r = z1 ? r2 : r1;
+    const double o = r * fma(z1 ? negF(grad) : grad, (z1 ? r4 : r3) - half(r), rv);
+    o1 = z1 ? 0.0 : o;
+    o2 = z1 ? o : 0.0;
+    return;
+  }
+#endif
   o1 = r1 * (rv + grad * (r3 - half(r1)));
   o2 = r2 * (rv - grad * (r4 - half(r2)));
-#endif
 }
 
 // ================================================================ k_ale_flux
