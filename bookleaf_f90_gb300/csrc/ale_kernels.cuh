@@ -198,8 +198,8 @@ __device__ __forceinline__ void elvl_pair(int i1, const int* nb, const int* fc,
 
 // LOOP: k_lag_state of the same step left the swept volumes of every
 // element's faces 0 and 3; a face 1 or 2 takes the one of the face across it
-// when that is a face 0 or 3 (exactly the negative), so 12 FP64 operations a
-// face are done once: Noh 1024x1024 1047 -> 997 us a step (with k_lag_state's
+// when that is a face 0 or 3 of the same nodes (exactly the negative), so 12
+// FP64 operations a face are done once: Noh 1024x1024 1047 -> 997 us a step (with k_lag_state's
 // unread results left out), the demoted form 981 -> 931, a 97x97 blast 64 -> 60.
 template <int BS, bool BATCH, bool LOOP>
 __global__ void __launch_bounds__(BS) k_ale_flux(DevFields F, DevCfg C) {
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(BS) k_ale_flux(DevFields F, DevCfg C) {
     fv[3] = F.fdv3[iel];
 #pragma unroll
     for (int j = 1; j <= 2; j++) {
-      if (nb[j] != iel && (fc[j] == 0 || fc[j] == 3)) {
+      if (swept_across(fcp, j)) {
         fv[j] = negF((fc[j] == 0 ? F.fdv0 : F.fdv3)[nb[j]]);
       } else {
         const int a = n[j], b = n[j + 1];

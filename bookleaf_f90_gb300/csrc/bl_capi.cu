@@ -536,6 +536,7 @@ int init_impl(bl_ctx** out, const bl_sizes* sizes, const bl_config* config, void
       su::k_sort<<<gn, su::kThreads, 0, x->stream>>>(d_off, nullptr, nel, nnd, d_ent2);
       F.ne_off = d_off;
       F.ne_ent = d_ent2;
+      su::k_swept_faces<<<ge, su::kThreads, 0, x->stream>>>(d_nd, d_ee, d_fc, nel);
     }
     // the edges' slots, for the build that computes an edge once; how many
     // there are is known at the next wait

@@ -84,7 +84,7 @@ struct DevFields {
   // connectivity (0-based)
   const int4* ielnd;
   const int4* ielel;
-  const int* ielfc;          // 4 x 8-bit face numbers 0..3
+  const int* ielfc;          // 4 x 8 bits: face number 0..3, kSweptAcross
   const int* ielreg;         // 0-based region
   const int* ielmat;         // material (<=0: mixed / void)
   const int* indtype;
@@ -176,7 +176,13 @@ __device__ __forceinline__ double minF_nn(double a, double b) { return gt_nn(a, 
 // Fortran SIGN(a,b): |a| with the sign bit of b (negative zero honoured);
 // signF itself is in bl_fp64.cuh, a sign-bit operation.
 
-__device__ __forceinline__ int fc_of(int packed, int j) { return (packed >> (8 * j)) & 0xff; }
+__device__ __forceinline__ int fc_of(int packed, int j) { return (packed >> (8 * j)) & 3; }
+// set beside the number of a face 1 or 2 whose nodes the element across holds
+// as its face 0 or 3, the other way round (k_swept_faces)
+constexpr int kSweptAcross = 0x80;
+__device__ __forceinline__ bool swept_across(int packed, int j) {
+  return (packed >> (8 * j)) & kSweptAcross;
+}
 
 __device__ __forceinline__ double c4(const d4& v, int j) {
   return j == 0 ? v.x : (j == 1 ? v.y : (j == 2 ? v.z : v.w));

@@ -234,6 +234,26 @@ __device__ __forceinline__ int at4(const int4& v, int j) {
 }
 __device__ __forceinline__ int face_byte(int packed, int j) { return (packed >> (8 * j)) & 3; }
 
+// Marks (bit 0x80 << 8 f) the faces f = 1, 2 whose nodes the element across
+// holds as its face 0 or 3, the other way round: the volume such a face sweeps
+// is exactly the negative of the one across, whichever way the connectivity
+// leads back.
+__global__ void __launch_bounds__(kThreads)
+    k_swept_faces(const int4* __restrict__ nd, const int4* __restrict__ ee, int* __restrict__ fc,
+                  int nel) {
+  const int e = blockIdx.x * kThreads + threadIdx.x;
+  if (e >= nel) return;
+  const int4 n = nd[e], nb = ee[e];
+  int v = fc[e];
+  for (int f = 1; f <= 2; f++) {
+    const int g = face_byte(v, f);
+    const int4 m = nd[at4(nb, f)];
+    if ((g == 0 || g == 3) && at4(m, g) == at4(n, f + 1) && at4(m, (g + 1) & 3) == at4(n, f))
+      v |= 0x80 << (8 * f);
+  }
+  fc[e] = v;
+}
+
 // the nodes of the two faces that continue face f of element e, or the
 // boundary rule's ratio there (kEndWall: 0, kEndMirror: 1) in both entries
 struct EdgeEnds {
