@@ -6,6 +6,7 @@
 // way inf_solver_getdt / inf_solver_lagstep / inf_solver_alestep sequence
 // the reference's loops.  No CPU fallback exists: every entry point fails
 // when CUDA is not usable.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1135,14 +1136,33 @@ __global__ void __launch_bounds__(256) k_move(const __grid_constant__ MoveTable 
   }
 }
 
-// whether a kernel may address this host array: pinned memory
-bool pinned(const void* p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return a.type == cudaMemoryTypeHost && a.devicePointer == p;
+// Whether a kernel may address this host array of n doubles: pinned memory,
+// all of it in one allocation or registration.  (A host may have registered a
+// part of the array only; the copies leave that to the runtime.)
+bool pinned(const void* p, size_t n) {
+  using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Query query = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault,
+                                         &found) != cudaSuccess) {
+      cudaGetLastError();
+      return Query(nullptr);
+    }
+    return found == cudaDriverEntryPointSuccess ? reinterpret_cast<Query>(f) : nullptr;
+  }();
+  if (!query) return false;
+  CUpointer_attribute want[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                 CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                 CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  unsigned type = 0, managed = 0;
+  CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p), device = 0, start = 0;
+  size_t size = 0;
+  void* got[5] = {&type, &managed, &device, &start, &size};
+  if (query(5, want, got, at) != CUDA_SUCCESS) return false;
+  return type == CU_MEMORYTYPE_HOST && !managed && device == at && at >= start &&
+         size >= at - start && n <= (size - (at - start)) / sizeof(double);
 }
 
 class Mover {
@@ -1180,7 +1200,7 @@ class Mover {
 // the host arrays are pinned; false where they are not.
 bool queue_move(bl_ctx* x, Mover& mv, int id, double* d, size_t n) {
   if (x->ninst == 0) {
-    if (!pinned(x->host[id])) return false;
+    if (!pinned(x->host[id], n)) return false;
     mv.add(d, static_cast<double*>(x->host[id]), n);
     return true;
   }
@@ -1514,7 +1534,7 @@ void batch_copy(bl_ctx* x, int id, bool to_mesh) {
 // none, otherwise.
 bool batch_moves(bl_ctx* x, int id, const std::function<void(void*, size_t, size_t)>& piece) {
   bool all = true;
-  batch_pieces(x, id, [&](void* mine, size_t, size_t) { all = all && pinned(mine); });
+  batch_pieces(x, id, [&](void* mine, size_t, size_t n) { all = all && pinned(mine, n); });
   if (all) batch_pieces(x, id, piece);
   return all;
 }
