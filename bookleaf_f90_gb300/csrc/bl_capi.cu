@@ -15,6 +15,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <utility>
 #include <vector>
 
 #include "../../include/bookleaf_gb300.h"
@@ -60,8 +61,10 @@ const bl::Launchers kMixed = {bl::mixed::getdt_blocks,          bl::mixed::getdt
 
 // batches (defined with bl_init_batch below)
 void batch_copy(bl_ctx* x, int id, bool to_mesh);
-bool batch_moves(bl_ctx* x, int id, const std::function<void(void*, size_t, size_t)>& piece);
-
+using Piece = std::function<void(void*, size_t, size_t)>;  // array, first value, values
+void batch_pieces(bl_ctx* x, int id, const Piece& piece);
+bool batch_moves(bl_ctx* x, int id, const Piece& piece);
+size_t state_count(const bl_ctx* x, int id);
 
 void set_err(bl_error* e, int ierr, int iout, const char* msg) {
   if (!e) return;
@@ -1196,9 +1199,32 @@ class Mover {
   MoveTable T_;
 };
 
+// Whether any two of the context's registered state arrays share memory.  The
+// moves of one launch come in no order; copies, one after the other, leave
+// what the last of them wrote.  (The arrays are those of the set-up: asked once.)
+bool arrays_overlap(bl_ctx* x) {
+  if (x->overlap < 0) {
+    std::vector<std::pair<const char*, const char*>> r;
+    auto add = [&](void* p, size_t, size_t n) {
+      const char* c = static_cast<const char*>(p);
+      if (c && n) r.emplace_back(c, c + n * sizeof(double));
+    };
+    for (int id : kStateIds) {
+      if (x->ninst > 0) batch_pieces(x, id, add);
+      else add(x->host[id], 0, state_count(x, id));
+    }
+    std::sort(r.begin(), r.end());
+    x->overlap = 0;
+    for (size_t i = 1; i < r.size(); i++)
+      if (r[i].first < r[i - 1].second) x->overlap = 1;
+  }
+  return x->overlap != 0;
+}
+
 // Queues the copy of field id (n doubles at d on the device) in `mv` where
 // the host arrays are pinned; false where they are not.
 bool queue_move(bl_ctx* x, Mover& mv, int id, double* d, size_t n) {
+  if (arrays_overlap(x)) return false;
   if (x->ninst == 0) {
     if (!pinned(x->host[id], n)) return false;
     mv.add(d, static_cast<double*>(x->host[id]), n);
@@ -1244,6 +1270,17 @@ static size_t field_count(const bl_ctx* x, int id, int& kind) {
       return 0;
   }
 }
+
+}  // extern "C"
+namespace {
+// values of a state field's host array (0: not one)
+size_t state_count(const bl_ctx* x, int id) {
+  int kind;
+  const size_t n = field_count(x, id, kind);
+  return kind < 0 ? 0 : n;
+}
+}  // namespace
+extern "C" {
 
 static void* dev_ptr(bl_ctx* x, int id) {
   bl::DevFields& F = x->F;
@@ -1505,8 +1542,7 @@ bool same_shared(const bl_config& a, const bl_config& b) {
 
 // Calls piece(mesh's own registered array, first value in the concatenated
 // field, values) for every mesh that has values of field id.
-template <class F>
-void batch_pieces(bl_ctx* x, int id, F piece) {
+void batch_pieces(bl_ctx* x, int id, const Piece& piece) {
   const FieldLayout L = field_layout(id);
   if (L.layout == kLayNone || L.is_int || !x->host[id]) return;
   const std::vector<int>& off = L.layout == kLayNd ? x->nd_off
@@ -1532,7 +1568,7 @@ void batch_copy(bl_ctx* x, int id, bool to_mesh) {
 
 // The pieces of field id when every mesh's own array is pinned; false, and
 // none, otherwise.
-bool batch_moves(bl_ctx* x, int id, const std::function<void(void*, size_t, size_t)>& piece) {
+bool batch_moves(bl_ctx* x, int id, const Piece& piece) {
   bool all = true;
   batch_pieces(x, id, [&](void* mine, size_t, size_t n) { all = all && pinned(mine, n); });
   if (all) batch_pieces(x, id, piece);

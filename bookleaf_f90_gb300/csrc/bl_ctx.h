@@ -27,6 +27,7 @@ struct bl_ctx {
   double* cn_gather = nullptr;  // [2][4*nel]: cnx, cny gathered for bl_sync_to_host
   bl::DevStep* hstep = nullptr;  // pinned mirror of F.step
   int* hgeom = nullptr;          // pinned, behind it: k_check_geometry's answer
+  int overlap = -1;              // two registered state arrays share memory (-1: not asked)
   // true while *hstep equals F.step on the device: set by a completed
   // fetch of the header, cleared whenever work that may change it is queued
   bool hstep_current = false;
