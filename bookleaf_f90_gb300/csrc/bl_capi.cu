@@ -925,7 +925,7 @@ int bl_run(bl_ctx* x, bl_timestep* ts, int max_steps, bl_step_record* history, i
   F.loop_ale = with_ale;
   const int G = 16;  // steps per graph launch
   if (!x->gexec || x->gsteps != G || x->g_ale != with_ale || x->g_hist != F.hist ||
-      x->g_maxrec != C.max_records) {
+      x->g_maxrec != C.max_records || x->g_geom != F.geom_x) {
     if (x->gexec) cudaGraphExecDestroy(x->gexec);
     x->gexec = nullptr;
     cudaGraph_t g;
@@ -947,6 +947,7 @@ int bl_run(bl_ctx* x, bl_timestep* ts, int max_steps, bl_step_record* history, i
     x->g_ale = with_ale;
     x->g_hist = F.hist;
     x->g_maxrec = C.max_records;
+    x->g_geom = F.geom_x;
   }
   header_from_ts(x, ts, 1);
   // step limit: getdt stops once nrecord reaches it (DevStep.nrecord counts)
@@ -1389,17 +1390,6 @@ int bl_sync_to_host(bl_ctx* x, int id) {
   return BL_SUCCESS;
 }
 
-// The answer of k_check_geometry.  The device loops' graphs hold the flag as
-// it was at their capture (the called entry points' are keyed on it).
-static void set_geom_x(bl_ctx* x, int v) {
-  if (x->F.geom_x == v) return;
-  x->F.geom_x = v;
-  if (x->gexec) cudaGraphExecDestroy(x->gexec);
-  x->gexec = nullptr;
-  if (x->bexec) cudaGraphExecDestroy(x->bexec);
-  x->bexec = nullptr;
-}
-
 static void queue_upload(bl_ctx* x, Mover& mv, int id) {
   if (id < 1 || id > BL_NID || !x->host[id]) return;
   int kind;
@@ -1420,7 +1410,7 @@ static int finish_upload(bl_ctx* x, Mover& mv, bool cs2, bool geometry) {
                     x->s.nel * sizeof(double), cudaMemcpyDeviceToDevice, x->stream);
   cudaError_t r = cudaStreamSynchronize(x->stream);
   if (r == cudaSuccess) r = cudaGetLastError();
-  if (geometry) set_geom_x(x, r == cudaSuccess ? *x->hgeom : 1);
+  if (geometry) x->F.geom_x = r == cudaSuccess ? *x->hgeom : 1;  // the graphs are keyed on it
   return r == cudaSuccess ? BL_SUCCESS : BL_FAILURE;
 }
 
@@ -1831,7 +1821,8 @@ int bl_run_batch(bl_ctx* x, bl_timestep* ts, int max_steps, int* status, int* ns
     queue_state(x, x->L.lag_state_b, x->L.mix_closure_b, F, C);
     if (with_ale) x->L.ale_b(F, C, x->stream);
   };
-  if (!x->bexec || x->b_ale != with_ale || x->b_gsteps != G || x->b_ndblock != F.nd_block) {
+  if (!x->bexec || x->b_ale != with_ale || x->b_gsteps != G || x->b_ndblock != F.nd_block ||
+      x->b_geom != F.geom_x) {
     if (x->bexec) cudaGraphExecDestroy(x->bexec);
     x->bexec = nullptr;
     cudaGraph_t g;
@@ -1849,6 +1840,7 @@ int bl_run_batch(bl_ctx* x, bl_timestep* ts, int max_steps, int* status, int* ns
     x->b_ale = with_ale;
     x->b_gsteps = G;
     x->b_ndblock = F.nd_block;
+    x->b_geom = F.geom_x;
   }
   const int per_step = x->L.getdt_launches(x->C) + bl::launches_lagstep(x->F) + (with_ale ? bl::kLaunchesAle : 0);
   int done = 0;

@@ -53,13 +53,13 @@ struct bl_ctx {
   cudaGraphExec_t bexec = nullptr;             // graph of batch steps
   bool b_ale = false;
   int b_graph_steps = 16;                      // steps per graph (autotuned)
-  int b_gsteps = 0, b_ndblock = 0;             // what bexec was captured with
+  int b_gsteps = 0, b_ndblock = 0, b_geom = 0;  // what bexec was captured with
   // bl_run
   cudaGraphExec_t gexec = nullptr;
   int gsteps = 0;
   bool g_ale = false;
   bl::StepRec* g_hist = nullptr;  // history buffer and record limit the
-  int g_maxrec = -1;              // graph's kernel arguments were captured with
+  int g_maxrec = -1, g_geom = 0;  // graph's kernel arguments were captured with
   int hist_cap = 0;
   std::vector<int> ielmat_h;  // for timestep%mdt
   // diagnostics scratch (bl_shortprint, bl_check_sod), grown on demand
