@@ -3,10 +3,9 @@
 // Four kernels per ALE step replace the reference's loops of
 // inf_solver_alestep (inf_solver_alestep.f90:39-74):
 //   k_ale_flux    ale_kn_getmeshvelocity + geometry_kn_getvertex +
-//                 geometry_kn_getfluxvolume (flux volume of every face; the
-//                 neighbour's value for a shared face is minus the own one
-//                 before the cut, so the volume sum needs no second pass),
-//                 ale_kn_sumflux(fcdv) and the mass flux ale_kn_fluxelvl.
+//                 geometry_kn_getfluxvolume (flux volume of every face) and the
+//                 mass flux ale_kn_fluxelvl (ale_kn_sumflux(fcdv)'s sum is read
+//                 by nothing).
 //   k_ale_el      ale_kn_sumflux(fcdm), ale_kn_updatebasisel, the energy flux
 //                 ale_kn_fluxelvl, ale_kn_fluxbasisnd (corner mass fluxes)
 //                 and both momentum passes of ale_kn_fluxndvl.
@@ -91,23 +90,21 @@ __device__ __forceinline__ double grad_f32(double A, double B, double mA, double
 #endif
 
 #if BL_FAST_ALGEBRA && !BL_MIXED
-// neither infinite nor a NaN; that and above zero
+// neither infinite nor a NaN
 __device__ __forceinline__ bool finiteF(double x) {
   return ((unsigned)(bits64(x) >> 32) & 0x7ff00000u) != 0x7ff00000u;
 }
-__device__ __forceinline__ bool positiveF(double x) {
-  return (unsigned long long)bits64(x) - 1 < 0x7fefffffffffffffull;
+// the leading words of an absolute value and of a value, and whether one is
+// that of a positive normal number
+__device__ __forceinline__ unsigned habs(double x) {
+  return (unsigned)(bits64(x) >> 32) & 0x7fffffffu;
 }
+__device__ __forceinline__ unsigned hword(double x) { return (unsigned)(bits64(x) >> 32); }
+__device__ __forceinline__ bool normal_word(unsigned h) { return h - 0x00100000u < 0x7fe00000u; }
 // -1, 0 or 1 for a * b below, near (within 2^-18) or above c * d, from the
-// leading 21 bits and the exponents, on the integer pipe; 0 also for zero and
-// subnormal operands.  Signs are ignored, no operand is infinite or a NaN.
-__device__ __forceinline__ int order_products(double a, double b, double c, double d) {
-  const unsigned ha = (unsigned)(bits64(a) >> 32) & 0x7fffffffu;
-  const unsigned hb = (unsigned)(bits64(b) >> 32) & 0x7fffffffu;
-  const unsigned hc = (unsigned)(bits64(c) >> 32) & 0x7fffffffu;
-  const unsigned hd = (unsigned)(bits64(d) >> 32) & 0x7fffffffu;
-  const unsigned lo = 0x00100000u;  // a normal number's at least
-  if (ha < lo || hb < lo || hc < lo || hd < lo) return 0;
+// leading words of four positive normal numbers, on the integer pipe
+__device__ __forceinline__ int order_products(unsigned ha, unsigned hb, unsigned hc, unsigned hd) {
+  const unsigned lo = 0x00100000u;
   const int e = (int)(ha >> 20) + (int)(hb >> 20) - (int)(hc >> 20) - (int)(hd >> 20);
   if (e > 2 || e < -2) return e > 0 ? 1 : -1;
   const unsigned long long p =
@@ -129,8 +126,8 @@ __device__ __forceinline__ int order_products(double a, double b, double c, doub
 // smaller of those two quotients, and which one that is shows in the
 // products A mB and B mA: one divide, no product in the FP64 pipe, where
 // the three candidates took three divides and seven operations.  (Two
-// divides when the products are too near to tell.)  Masses of other signs,
-// infinities and NaN take the three candidates.
+// divides when the products are too near to tell.)  Masses that are not
+// positive, subnormal numbers, infinities and NaN take the three candidates.
 __device__ __forceinline__ double slope_of_three(double A, double B, double mA, double mB,
                                                  double S) {
   const double w8 = DIV(A * mB * mB + B * mA * mA, mA * mB * (mA + mB));
@@ -145,8 +142,9 @@ __device__ __forceinline__ double limited_slope(double A, double B, double mA, d
 #else
 #if BL_FAST_ALGEBRA
   if (prod_le0(A, B)) return 0.0;
-  if (finiteF(A) && finiteF(B) && positiveF(mA) && positiveF(mB)) {
-    const int o = order_products(A, mB, B, mA);
+  const unsigned hA = habs(A), hB = habs(B), hmA = hword(mA), hmB = hword(mB);
+  if (normal_word(hA) && normal_word(hB) && normal_word(hmA) && normal_word(hmB)) {
+    const int o = order_products(hA, hmB, hB, hmA);
     const double q = DIV(absF(o > 0 ? B : A), o > 0 ? mB : mA);
     return signF(o == 0 ? minF_nn(q, DIV(absF(B), mB)) : q, S);
   }
@@ -155,34 +153,46 @@ __device__ __forceinline__ double limited_slope(double A, double B, double mA, d
 #endif
 }
 
+// whether neither an infinity nor a NaN is among a value and four corners'
+__device__ __forceinline__ bool all_finite(double v, const d4& c) {
+#if BL_FAST_ALGEBRA && !BL_MIXED
+  const unsigned x = max(max(habs(v), max(habs(c.x), habs(c.y))), max(habs(c.z), habs(c.w)));
+  return x < 0x7ff00000u;
+#else
+  return true;
+#endif
+}
+
 // The limited face flux of ale_kn_fluxelvl for the pair (i1, i2=i1+2),
 // returning (fcflux(i1), fcflux(i2)) (ale_kn_advectors.f90:48-78).
 // Fast build: where nothing leaves through a face its flux is 0 without the
 // arithmetic -- unless that would be 0 times an infinity or a NaN, which the
-// neighbour has to meet.
+// neighbour has to meet (finite: rv and own_b have neither).
 __device__ __forceinline__ void elvl_pair(int i1, const int* nb, const int* fc,
                                           const d4* cnbasis, const double* own_b,
                                           double r1, double r2, const double* elvar,
-                                          double rv, double& o1, double& o2) {
+                                          double rv, bool finite, double& o1, double& o2) {
   const int i2 = i1 + 2;
   const int iel1 = nb[i1], iel2 = nb[i2];
-  const double w1 = rv - elvar[iel2], w2 = elvar[iel1] - rv;
-  const double r3 = own_b[i2] + own_b[(i2 + 1) & 3], r4 = own_b[i1] + own_b[i1 + 1];
+  const double e1 = elvar[iel1], e2 = elvar[iel2];
 #if BL_FAST_ALGEBRA && !BL_MIXED
-  // nothing leaves through either face (fluid at rest), and no slope
+  // nothing leaves through either face, and one side has the same value, which
+  // makes the slope 0 (fluid at rest; on bit patterns alone)
   const bool z1 = (bits64(r1) << 1) == 0, z2 = (bits64(r2) << 1) == 0;
-  if (z1 && z2 && prod_le0(w1, w2) && finiteF(rv) && finiteF(r3) && finiteF(r4)) {
+  if (z1 && z2 && finite && (bits64(e1) == bits64(rv) || bits64(e2) == bits64(rv))) {
     o1 = o2 = 0.0;
     return;
   }
 #endif
+  const double w1 = rv - e2, w2 = e1 - rv;
+  const double r3 = own_b[i2] + own_b[(i2 + 1) & 3], r4 = own_b[i1] + own_b[i1 + 1];
   const int f1 = fc[i1], f2 = fc[i2];
   const double w5 = r3 + cget(cnbasis, iel2, f2) + cget(cnbasis, iel2, (f2 + 1) & 3);
   const double w6 = r4 + cget(cnbasis, iel1, f1) + cget(cnbasis, iel1, (f1 + 1) & 3);
   const double grad = limited_slope(w1, w2, w5, w6, w2);
 #if BL_FAST_ALGEBRA && !BL_MIXED
   // flow through the pair leaves through one face; the other's flux is 0
-  if ((z1 || z2) && finiteF(grad) && finiteF(rv) && finiteF(r3) && finiteF(r4)) {
+  if ((z1 || z2) && finite && finiteF(grad)) {
     const double r = z1 ? r2 : r1;
     const double o = r * fma(z1 ? negF(grad) : grad, (z1 ? r4 : r3) - half(r), rv);
     o1 = z1 ? 0.0 : o;
@@ -267,9 +277,10 @@ __global__ void __launch_bounds__(BS) k_ale_flux(DevFields F, DevCfg C) {
   const d4 cw = F.cnwt[iel];
   const double ob[4] = {cw.x, cw.y, cw.z, cw.w};
   const double rv = F.rho[iel];
+  const bool fin = all_finite(rv, cw);
   double fm[4];
-  elvl_pair(0, nb, fc, F.cnwt, ob, fv[0], fv[2], F.rho, rv, fm[0], fm[2]);
-  elvl_pair(1, nb, fc, F.cnwt, ob, fv[1], fv[3], F.rho, rv, fm[1], fm[3]);
+  elvl_pair(0, nb, fc, F.cnwt, ob, fv[0], fv[2], F.rho, rv, fin, fm[0], fm[2]);
+  elvl_pair(1, nb, fc, F.cnwt, ob, fv[1], fv[3], F.rho, rv, fin, fm[1], fm[3]);
   F.fcdm[iel] = make_d4(fm[0], fm[1], fm[2], fm[3]);
 }
 
@@ -282,7 +293,6 @@ __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
   const int4 ee = __ldg(F.ielel + iel);
   DevStep* S = el_step<BATCH>(F, iel);
   if (halted_a(S) || !ale_on(C, S)) return;
-  const double zc = C.zerocut;
   const int nb[4] = {ee.x, ee.y, ee.z, ee.w};
   const int fcp = __ldg(F.ielfc + iel);
   const int fc[4] = {fc_of(fcp, 0), fc_of(fcp, 1), fc_of(fcp, 2), fc_of(fcp, 3)};
@@ -343,9 +353,10 @@ __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
   const d4 cm = F.cnmass[iel];
   const double ob[4] = {cm.x, cm.y, cm.z, cm.w};
   const double ev = F.e[iel];
+  const bool fin = all_finite(ev, cm);
   double ef[4];
-  elvl_pair(0, nb, fc, F.cnmass, ob, fm[0], fm[2], F.e, ev, ef[0], ef[2]);
-  elvl_pair(1, nb, fc, F.cnmass, ob, fm[1], fm[3], F.e, ev, ef[1], ef[3]);
+  elvl_pair(0, nb, fc, F.cnmass, ob, fm[0], fm[2], F.e, ev, fin, ef[0], ef[2]);
+  elvl_pair(1, nb, fc, F.cnmass, ob, fm[1], fm[3], F.e, ev, fin, ef[1], ef[3]);
   F.eflux[iel] = make_d4(ef[0], ef[1], ef[2], ef[3]);
   // ale_kn_fluxndvl for u and v (ale_kn_advectors.f90:83-153): corner flux
   // pairs (ilndl, ilndr, ii) in loop order (ilfcl, icn) = (1,1),(1,2),(2,1),(2,2)
@@ -474,7 +485,6 @@ __global__ void __launch_bounds__(BS) k_ale_el(DevFields F, DevCfg C) {
   F.cnfu[iel] = make_d4(fu[0], fu[1], fu[2], fu[3]);
   F.cnfv[iel] = make_d4(fv[0], fv[1], fv[2], fv[3]);
 #endif
-  (void)zc;
 }
 
 // ================================================================ k_ale_nd
