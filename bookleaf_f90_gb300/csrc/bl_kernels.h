@@ -50,7 +50,7 @@ struct Launchers {
   void (*lag_accel_b)(const DevFields&, const DevCfg&, cudaStream_t);
   void (*lag_state_b)(const DevFields&, const DevCfg&, cudaStream_t);
   void (*ale_b)(const DevFields&, const DevCfg&, cudaStream_t);
-  // the learned mixed-cell closure (after lag_state; no-op when off)
+  // the learned mixed-cell closure (beside lag_state; no-op when off)
   int (*mix_prepare)();
   void (*mix_closure)(const DevFields&, const DevCfg&, cudaStream_t);
   void (*mix_closure_b)(const DevFields&, const DevCfg&, cudaStream_t);

@@ -88,14 +88,18 @@ static __device__ __noinline__ double dsqrt_call(double x) { return dsqrt_rn(x);
 #endif
 
 // Resident blocks per SM that the edge and candidate kernels (of 128 threads)
-// and k_lag_force (of 64) are compiled for.  All are bound by the FP64 pipe,
-// which two or three warps a scheduler fill as long as their integer divide
-// chains overlap, so the bound is the register count that spills nothing.
+// and k_lag_force (of 64) are compiled for.  All are bound by the FP64 pipe and
+// wait for their integer divide chains, so warps pay until their registers run
+// out: k_lag_force spills nothing at its bound, k_getdt is still faster with
+// some 60 spilled values a zone at 7 blocks than without at 4.
 // k_getdt at 4/5/6/7/8 blocks: Sedov 512x512 (with the edge kernel)
-// 75/73/72/69/69 us.  k_lag_force at 3/4/5/6 blocks of 128: 100/90/90/91 us
-// with sub-zonal and hourglass forces; five is faster by 8 % where the mesh
-// fits one wave of five and not of four (280x280 to 301x301) and slower by 6
-// to 9 % at 200x200, 330x330 and 450x450.
+// 75/73/72/69/69 us; k_edge at 6/7/10/12 within 1 us of 8.  k_lag_force in
+// blocks of 128, before they became 64, at 3/4/5/6: 100/90/90/91 us with
+// sub-zonal and hourglass forces; five was faster by 8 % where the mesh fits one
+// wave of five and not of four (280x280 to 301x301) and slower by 6 to 9 % at
+// 200x200, 330x330 and 450x450.  In blocks of 64 at twice the bound (the
+// registers are the same) the last wave is finer: a step of 200x200 54.7 -> 50.9
+// us, of 512x512 187.6 -> 185.3 (with k_lag_state in blocks of 64 too).
 #ifndef BL_GETDT_MINB
 #define BL_GETDT_MINB 7
 #endif
@@ -872,16 +876,19 @@ __device__ __forceinline__ void getdt_finish(const DevFields& F, const DevCfg& C
 
 // Consecutive tiles of BS elements that a k_getdt block of the fast and mixed
 // builds takes, for nel elements in all meshes together: about as many blocks
-// as are resident at once (152 SMs of 7), at least one tile and at most 8.  A
-// block ends with a barrier and a ticket of a microsecond, which 8,192 blocks
-// of one tile each pay one after another on every SM: Noh 1024x1024, 1, 2, 4,
-// 8 and 16 tiles, the mixed build's k_edgevisc + k_getdt 203, 190, 180, 172,
-// 196 us, the fast build's pair 261, 259, 258, 259, 280; Sedov 512x512 (2,048
-// tiles) 1, 2 and 4 tiles 65.3, 63.6, 67.6 us; fewer than 1.5 tiles a resident
-// block are better left one each.
+// as are resident at once (152 SMs of BL_GETDT_MINB), at least one tile and at
+// most 8.  A block ends with a barrier and a ticket of a microsecond, which
+// 8,192 blocks of one tile each pay one after another on every SM: Noh
+// 1024x1024, 1, 2, 4, 8 and 16 tiles, the mixed build's k_edgevisc + k_getdt
+// 203, 190, 180, 172, 196 us.  The fast build's k_getdt has FP64 work to hide
+// them behind (its pair 261, 259, 258, 259, 280): the rule is the mixed
+// build's, and costs the fast one nothing.  Sedov 512x512 (2,048 tiles) 1, 2
+// and 4 tiles 65.3, 63.6, 67.6 us; fewer than 1.5 tiles a resident block are
+// better left one each.
 __host__ __device__ __forceinline__ int getdt_tiles(int nel, int bs) {
   if (!BL_FAST_ALGEBRA) return 1;
-  const int t = (nel / bs + 532) / 1064;
+  constexpr int resident = 152 * BL_GETDT_MINB;
+  const int t = (nel / bs + resident / 2) / resident;
   return t < 1 ? 1 : (t > 8 ? 8 : t);
 }
 
@@ -1789,11 +1796,11 @@ __global__ void __launch_bounds__(BS, BL_GETDT_MINB) k_getdt(DevFields F, DevCfg
 //   and their work, with q_j = spmass_j / V_j,
 //     pmerit cs2 / 8 (2 Dv (sum q_j - 4 rho) + B (q0 - q2) - C (q1 - q3)),
 //     B = d h - 2 b2 U13 - (y), C = s h + 2 b2 U02 - (y).
-// 140 FP64 instructions an element with all forces on where the reference's
-// terms one by one took 206, and no corner positions gathered: Sedov
-// 512x512 108 -> 90 us (FP64 pipe 79 % busy over the SMs' active cycles, the
-// divide chains' latency the rest; 3, 5 and 6 blocks per SM and blocks of 64
-// and 256 threads are slower or equal), 42 -> 39 us at 90,000 elements.
+// 152 FP64 instructions an element in motion with all forces on where the
+// reference's terms one by one took 206, and no corner positions gathered:
+// Sedov 512x512 108 -> 88 us, 42 -> 39 us at 90,000 elements; FP64 pipe 71 %
+// busy over the SMs' active cycles, the divide chains' latency the rest (blocks
+// and bound: BL_FORCE_MINB).
 // POS: where the coefficients or volumes are not those of the positions
 // (DevFields::geom_x), the half-step geometry and the sub-zonal pressures are
 // formed from the corners; the pressure force keeps the stored coefficients,

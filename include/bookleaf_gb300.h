@@ -205,7 +205,9 @@ int bl_run(bl_ctx *ctx, bl_timestep *timestep, int max_steps,
  * hydro_dr_shortprint).  id = 0 copies every registered state field. */
 int bl_sync_to_host(bl_ctx *ctx, int id);
 
-/* Uploads host field id again after the host changed it (id = 0: all). */
+/* Uploads host field id again after the host changed it (id = 0: all).  Node
+ * positions, the element coefficients a1..b3 and elvolume need not agree: the
+ * next step takes each quantity from where the reference takes it. */
 int bl_sync_to_device(bl_ctx *ctx, int id);
 
 /* ---- batches of meshes (no counterpart in the reference) ------------------
