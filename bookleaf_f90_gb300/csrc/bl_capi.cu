@@ -238,8 +238,11 @@ __global__ void __launch_bounds__(256) k_check_geometry(bl::DevFields F, int* di
 #pragma unroll
     for (int k = 0; k < 6; k++) bad = bad || !le_nn(absF(c[k] - s[k]), k < 3 ? tx : ty);
     const double q = a3 * b1, v = times4(fma(a1, b3, -q));
-    const long long units = bits64(v) - bits64(vol);
-    if (units > 8 || units < -8 || !gtF(HUGE_VAL, absF(v))) {
+    // (patterns of one sign next to each other: the wrapped difference of two
+    // signs is small only for a NaN)
+    const long long units =
+        (long long)((unsigned long long)bits64(v) - (unsigned long long)bits64(vol));
+    if (units > 8 || units < -8 || !gtF(HUGE_VAL, absF(v)) || !gtF(HUGE_VAL, absF(vol))) {
       const double tv = 4.0 * (tx * (fabs(b1) + fabs(b3)) + ty * (fabs(a1) + fabs(a3)) +
                                0x1p-49 * (fabs(a1 * b3) + fabs(q)));
       bad = bad || !(fabs(v - vol) <= tv);

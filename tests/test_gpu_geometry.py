@@ -162,3 +162,28 @@ def test_device_loops(build):
     for p, q in zip([one] + batch, [base[0]] + base):
         assert abs(p.timestep.dt - q.timestep.dt) <= tdt * q.timestep.dt
         _off(p, q, STEP, tol)
+
+
+@pytest.mark.parametrize("build", sorted(BUILDS))
+@pytest.mark.parametrize("value", [np.nan, np.inf, -0.0], ids=["nan", "inf", "minus_zero"])
+def test_a_volume_that_is_none(value, build):
+    """One cell's stored volume is no number, or zero: its half step and its
+    neighbours' are formed from the positions all the same."""
+    from oracle.oracle import Oracle
+    fp, tol, _ = BUILDS[build]
+    pc = _moving(DECKS["all_forces"])
+    before = pc.copy()
+    o = Oracle(pc)
+    assert o.getdt(pc.timestep) == 0
+    pc.fields[abi.ELVOLUME][5 * 12 + 5] = value
+    pg = before
+    s = Solver(pg, fp_mode=fp)
+    for f in pg.fields:
+        pg.fields[f][...] = pc.fields[f]
+    s.sync_to_device(0)
+    ts = pc.timestep.copy()
+    assert s.inf_solver_lagstep(ts) == o.lagstep(pc.timestep) == 0
+    s.sync_to_host(0)
+    s.close()
+    assert np.isfinite(pc.fields[abi.ELENERGY]).all()
+    _off(pg, pc, STEP, tol)
